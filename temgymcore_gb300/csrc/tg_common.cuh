@@ -37,6 +37,11 @@ enum OpKind : int32_t {
   OP_ABER = 10       // aberrated lens: c0 = 1/f, c1 = 1/(2f); aux = Program::aber slot
 };
 
+template <int K>
+struct OpConst {  // a step kind as a type: chain_forward_n specialises the step body on it
+  static constexpr int32_t value = K;
+};
+
 struct Op {
   int32_t kind;
   int32_t aux;   // OP_PROBE_SHIFT: index into Program::pcoef; OP_BIPRISM: sign-bit slot
@@ -101,8 +106,19 @@ __device__ __forceinline__ float sgnf(float v) {
 // decided by the float64 path, so the result equals the float64 result.
 struct BinCoef {
   float f[6];
+  float lim[2];  // 1/2 - 3 u |offset| - u, rows y and x (u = 2^-24)
   double d[6];
 };
+
+// With u = 2^-24, p0 = fl(m0 a), p1 = fl(m1 b + m2) and v = fl(p0 + p1): the
+// coefficients' float32 rounding and the product's cost 2 u |p0| and
+// u |m1 b| + u |m2|, the fused sum u |p1|, the last sum u |v|, and
+// |m1 b| <= |p1| + |m2|, so v is within u (3 (|p0| + |p1|) + 2 |m2|) of the
+// float64 value (to first order).  The test uses 4 u (|p0| + |p1|) + 3 u |m2|
+// + u; the last u covers the test's own rounding (2^-25 next to 1/2).  A bound
+// six times wider sent 12 % of the warps of a 512 x 512 detector to float64
+// per ray, 39 % of the float64 pipe.
+constexpr float kBinBound = 2.3841858e-07f;  // 4 u = 2^-22
 
 __device__ __forceinline__ int bin_exact64(float af, float bf, double m0,
                                            double m1, double m2) {
@@ -116,29 +132,47 @@ __device__ __forceinline__ int bin_exact64(float af, float bf, double m0,
   return __double2int_rn(v);  // cvt.rni.s32.f64: saturating
 }
 
-__device__ __forceinline__ int bin_one(float a, float b, float m0, float m1,
-                                       float m2, double d0, double d1,
-                                       double d2) {
-  float p0 = m0 * a, p1 = m1 * b;
-  float v = (p0 + p1) + m2;
-  float s = fabsf(p0) + fabsf(p1) + fabsf(m2);
-  // |v - exact| <= ~5 * 2^-24 * s; use 2^-19 * s (16x margin) + denormal guard
-  float bound = s * 1.9073486e-06f + 1e-30f;
+// One coordinate by the fast path; false: the float64 path has to decide.
+__device__ __forceinline__ bool bin_fast(float a, float b, float m0, float m1, float m2, float lim, int& out) {
+  const float p0 = m0 * a, p1 = fmaf(m1, b, m2);
+  const float v = p0 + p1;
   // nearest integer by the 1.5 * 2^23 constant (float32 ulp 1 there, exact
   // for |v| < 2^22), so no conversion instruction runs; r = v - rint(v)
-  // exactly, and 1/2 - |r| is the distance to the nearest half-integer
+  // exactly, and 1/2 - |r| is the distance to the nearest half-integer.  For
+  // |v| >= 2^22 and for non-finite terms the right-hand side is negative,
+  // infinite or NaN: never less.
   const float magic = 12582912.f;
   const float t = __fadd_rn(v, magic);
   const float r = __fsub_rn(v, __fsub_rn(t, magic));
-  bool ok = (fabsf(v) < 4194304.f) && (0.5f - fabsf(r) > bound);  // |v| < 2^22, finite
-  if (ok) return __float_as_int(t) - __float_as_int(magic);
-  return bin_exact64(a, b, d0, d1, d2);
+  out = __float_as_int(t) - __float_as_int(magic);
+  return fabsf(r) < fmaf(fabsf(p0) + fabsf(p1), -kBinBound, lim);
 }
 
-__device__ __forceinline__ void bin_yx(float x, float y, const BinCoef& bc,
-                                       int& py, int& px) {
-  py = bin_one(y, x, bc.f[0], bc.f[1], bc.f[2], bc.d[0], bc.d[1], bc.d[2]);
-  px = bin_one(y, x, bc.f[3], bc.f[4], bc.f[5], bc.d[3], bc.d[4], bc.d[5]);
+// R rays to pixel indices.  The fast paths of all R run straight through and
+// one branch serves them: a ray with an undecided coordinate takes the
+// float64 path for both.  nonfinite[k]: x or y is not finite (every such ray
+// takes the float64 path).
+template <int R>
+__device__ __forceinline__ void bin_rays(const float (&x)[R], const float (&y)[R], const BinCoef& bc,
+                                         int (&py)[R], int (&px)[R], bool (&nonfinite)[R]) {
+  bool ok[R], all = true;
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    const bool oky = bin_fast(y[k], x[k], bc.f[0], bc.f[1], bc.f[2], bc.lim[0], py[k]);
+    const bool okx = bin_fast(y[k], x[k], bc.f[3], bc.f[4], bc.f[5], bc.lim[1], px[k]);
+    ok[k] = oky & okx;
+    all &= ok[k];
+    nonfinite[k] = false;
+  }
+  if (!all) {
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+      if (!ok[k]) {
+        py[k] = bin_exact64(y[k], x[k], bc.d[0], bc.d[1], bc.d[2]);
+        px[k] = bin_exact64(y[k], x[k], bc.d[3], bc.d[4], bc.d[5]);
+        nonfinite[k] = !(isfinite(x[k]) && isfinite(y[k]));
+      }
+  }
 }
 
 inline BinCoef make_bincoef(const tg_grid* g) {
@@ -146,6 +180,10 @@ inline BinCoef make_bincoef(const tg_grid* g) {
   for (int i = 0; i < 6; ++i) {
     b.d[i] = g->m[i];
     b.f[i] = (float)g->m[i];
+  }
+  for (int i = 0; i < 2; ++i) {
+    const float o = b.f[3 * i + 2];
+    b.lim[i] = 0.5f - 0.75f * kBinBound * (o < 0.f ? -o : o) - 0.25f * kBinBound;
   }
   return b;
 }
@@ -392,6 +430,69 @@ __device__ __forceinline__ void op_forward(const Op& op, const float4* pshift,
     default:
       break;
   }
+}
+
+// One component applied to R independent rays: its free-space step f (the
+// compiler emits one before every component) and then its own step c, whose
+// kind is decided once for all R rays.  The arithmetic per ray is
+// op_forward's, expression for expression.
+template <int R>
+__device__ __forceinline__ void component_forward_n(const Op& f, const Op& c, bool varz, const float4* pshift,
+                                                    RayS (&r)[R], const float (&dvar)[R], uint64_t (&sbits)[R],
+                                                    bool (&alive)[R]) {
+  if (varz) {
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      r[k].x = fmaf(r[k].dx, dvar[k], r[k].x);
+      r[k].y = fmaf(r[k].dy, dvar[k], r[k].y);
+    }
+  } else {
+    const float d = f.c[0];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      r[k].x = fmaf(r[k].dx, d, r[k].x);
+      r[k].y = fmaf(r[k].dy, d, r[k].y);
+    }
+  }
+  auto all = [&](auto kind) {
+    Op o = c;
+    o.kind = decltype(kind)::value;
+#pragma unroll
+    for (int k = 0; k < R; ++k) op_forward(o, pshift, r[k], dvar[k], sbits[k], alive[k]);
+  };
+  if (c.kind == OP_NOP) return;
+  if (c.kind == OP_LENS) all(OpConst<OP_LENS>());
+  else if (c.kind == OP_SHIFT) all(OpConst<OP_SHIFT>());
+  else if (c.kind == OP_PROBE_SHIFT) all(OpConst<OP_PROBE_SHIFT>());
+  else if (c.kind == OP_DEFLECT) all(OpConst<OP_DEFLECT>());
+  else if (c.kind == OP_ROTATE) all(OpConst<OP_ROTATE>());
+  else if (c.kind == OP_APERTURE) all(OpConst<OP_APERTURE>());
+  else if (c.kind == OP_BIPRISM) all(OpConst<OP_BIPRISM>());
+}
+
+// The whole chain applied to R independent rays, component by component.
+// Chains with an aberrated lens or direction cosines keep the step loop.  (The
+// components unrolled, each step's coefficients at fixed constant-bank
+// addresses, ran slower: 105 instead of 89 us for 8 M rays through eight
+// components, 2.5 of 12 stalled cycles an issue waiting for instructions; a
+// switch instead of the comparisons 92.)
+template <int R>
+__device__ __forceinline__ void chain_forward_n(const Program& P, const float4* pshift, RayS (&r)[R],
+                                                const float (&dvar)[R], uint64_t (&sbits)[R], bool (&alive)[R],
+                                                const float* aber) {
+  if (P.dircos || P.n_aber > 0) {
+#pragma unroll 1
+    for (int s = 0; s < P.n_steps; ++s) {
+      const Op& op = P.op[s];
+#pragma unroll
+      for (int k = 0; k < R; ++k) op_forward(op, pshift, r[k], dvar[k], sbits[k], alive[k], aber);
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int s = 0; s < P.n_steps; s += 2)
+    component_forward_n<R>(P.op[s], P.op[s + 1], s == 0 && P.op[0].kind == OP_FREE_VARZ, pshift, r, dvar, sbits,
+                           alive);
 }
 
 // ---------------------------------------------------------------- adjoint

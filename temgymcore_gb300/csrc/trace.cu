@@ -22,7 +22,7 @@ struct FwdArgs {
   const double* z;
   double z_scalar;
   const double* pl;
-  double pl_scalar;
+  double pl_uniform;  // uniform input pathlength + the chain's uniform distances
   const float* amp;
   float *ox, *oy, *odx, *ody;
   double* opl;
@@ -132,23 +132,16 @@ __device__ __forceinline__ void store4(float* __restrict__ p, int64_t i0,
   }
 }
 
-struct NoOp {
-  __device__ __forceinline__ void operator()() const {}
-};
-
 // The chain, the outputs, the pixels and the histogram for rays i0 .. i0+R-1
 // whose inputs are in x, y, dx, dy (vec: all R in range and every output
 // array aligned for R-wide vector stores).  All 32 lanes of the warp call it
-// (the global histogram's warp aggregation).  after_chain runs once the
-// coordinates are stored (every input consumed), before the pathlength, the
-// binning and the histogram.
-template <int R, typename CountT, bool kSh, typename AfterChain = NoOp>
+// (the global histogram's warp aggregation).
+template <int R, typename CountT, bool kSh>
 __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, const BinCoef& B,
                                          uint32_t* shw, int64_t i0, float (&x)[R],
                                          float (&y)[R], float (&dx)[R], float (&dy)[R],
-                                         bool vec, AfterChain after_chain = AfterChain()) {
+                                         bool vec) {
   const int64_t n = A.n;
-  const double pl_uniform = A.pl_scalar + P.pl_const;
   {
     RayS r[R];
     double dvar[R];  // per-ray first distance (per-ray input z only), float64 once per ray
@@ -170,12 +163,7 @@ __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, con
         dvf[k] = (float)dvar[k];
       }
     }
-    for (int s = 0; s < P.n_steps; ++s) {
-      const Op op = P.op[s];
-#pragma unroll
-      for (int k = 0; k < R; ++k)
-        op_forward(op, nullptr, r[k], dvf[k], sb[k], alive[k], &P.aber[0][0]);
-    }
+    chain_forward_n<R>(P, nullptr, r, dvf, sb, alive, &P.aber[0][0]);
 #pragma unroll
     for (int k = 0; k < R; ++k) {
       x[k] = r[k].x; y[k] = r[k].y; dx[k] = r[k].dx; dy[k] = r[k].dy;
@@ -184,20 +172,24 @@ __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, con
     store4<R>(A.oy, i0, n, y, vec);
     store4<R>(A.odx, i0, n, dx, vec);
     store4<R>(A.ody, i0, n, dy, vec);
-    // every input value has reached an issued instruction (the output of each
-    // coordinate depends on its input), so their registers hold the data
-    after_chain();
     if (A.opl) {
       // no float64 arithmetic per ray for a uniform base (one add per
       // per-ray input): GB300 issues float64 at ~1/64 of the float32 rate,
-      // so base + plv is rounded with float32 / integer operations
+      // so base + plv is rounded with float32 / integer operations.  The two
+      // cases are separate loops: as selects on one loop's base the compiler
+      // ran the float64 adds for every ray (a quarter of the float64 pipe at
+      // 8 M rays through eight components, 88 -> 77 us without them)
       double o[R];
+      if (A.pl || A.z) {
 #pragma unroll
-      for (int k = 0; k < R; ++k) {
-        double base = pl_uniform;
-        if (A.pl && i0 + k < n) base = A.pl[i0 + k] + P.pl_const;
-        if (A.z) base += dvar[k];
-        o[k] = add_f64_f32(base, r[k].plv);
+        for (int k = 0; k < R; ++k) {
+          double base = A.pl && i0 + k < n ? A.pl[i0 + k] + P.pl_const : A.pl_uniform;
+          if (A.z) base += dvar[k];
+          o[k] = add_f64_f32(base, r[k].plv);
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < R; ++k) o[k] = add_f64_f32(A.pl_uniform, r[k].plv);
       }
       if (R == 4 && vec && A.opl_vec) {  // two 16-byte stores (i0 is a multiple of 4)
         reinterpret_cast<double2*>(A.opl + i0)[0] = make_double2(o[0], o[1]);
@@ -225,14 +217,13 @@ __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, con
     }
     if (A.do_bin) {
       int pys[R], pxs[R];
+      bool nonfinite[R];
+      bin_rays<R>(x, y, B, pys, pxs, nonfinite);
 #pragma unroll
       for (int k = 0; k < R; ++k) {
-        int py, px;
-        bin_yx(x[k], y[k], B, py, px);
-        pys[k] = py;
-        pxs[k] = px;
+        const int py = pys[k], px = pxs[k];
         const bool inr = (i0 + k < n);
-        if (inr && !(isfinite(x[k]) && isfinite(y[k]))) atomicOr(&g_tg_err, TG_EW_NONFINITE);
+        if (inr && nonfinite[k]) atomicOr(&g_tg_err, TG_EW_NONFINITE);
         if (A.hist) {
           bool ok = inr && alive[k] && py >= 0 && py < A.h && px >= 0 && px < A.w;
           if (kSh) hist_add_sh<CountT>(shw, ok ? py * A.w + px : 0, ok, reinterpret_cast<CountT*>(A.hist));
@@ -262,10 +253,10 @@ __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, con
 
 // kPf (shared-histogram variant, R = 4): each thread prefetches its next
 // four rays (x, y, dx, dy: four 16-byte cp.async) into its own 64-byte slot of
-// shared memory as soon as the current ones' coordinates are stored (every
-// value read from the slot has then been used), so the loads run under the
-// pathlength, the binning and the histogram atomics.  The slots take
-// kPfBytes ahead of the histogram words.
+// shared memory once the current ones are done.  Issued earlier, right behind
+// the coordinate stores, the reads mix with the pathlength and pixel writes and
+// the memory runs slower (16.8 M rays on 256 x 256: 163 us early, 144 here,
+// 145 without prefetching).  The slots take kPfBytes ahead of the histogram words.
 constexpr int kPfBytes = 4 * kShThreads * 16;  // 64 KB
 
 template <int R, typename CountT, bool kSh = false, bool kPf = false>
@@ -316,15 +307,11 @@ k_trace_fwd(const __grid_constant__ Program P, const __grid_constant__ FwdArgs A
       load4<R>(A.dx, i0, n, dx, vec);
       load4<R>(A.dy, i0, n, dy, vec);
     }
-    const int64_t ni0 = i0 + stride;
-    // the slot is free once the values read from it have been used
-    auto next = [&]() {
-      if (kPf) {
-        if (ni0 + 3 < n) prefetch(ni0);
-        cp_async_commit();
-      }
-    };
-    fwd_rays<R, CountT, kSh>(P, A, B, shw, i0, x, y, dx, dy, vec, next);
+    fwd_rays<R, CountT, kSh>(P, A, B, shw, i0, x, y, dx, dy, vec);
+    if (kPf) {  // the values read from the slot have been used
+      if (i0 + stride + 3 < n) prefetch(i0 + stride);
+      cp_async_commit();
+    }
   }
   if (kSh) sh_store_row(shw, A.rows + (size_t)blockIdx.x * sh_words(bins), sh_words(bins));
 }
@@ -401,13 +388,15 @@ k_bin(const __grid_constant__ BinArgs A, const __grid_constant__ BinCoef B) {
   for (int64_t blk = (int64_t)blockIdx.x * blockDim.x; blk < A.n; blk += stride) {
     const int64_t i = blk + threadIdx.x;
     const bool inr = i < A.n;
-    float x = inr ? A.x[i] : 0.f, y = inr ? A.y[i] : 0.f;
-    int py, px;
-    bin_yx(x, y, B, py, px);
+    const float x[1] = {inr ? A.x[i] : 0.f}, y[1] = {inr ? A.y[i] : 0.f};
+    int pys[1], pxs[1];
+    bool nonfinite[1];
+    bin_rays<1>(x, y, B, pys, pxs, nonfinite);
+    const int py = pys[0], px = pxs[0];
     if (inr) {
       if (A.pix_y) A.pix_y[i] = py;
       if (A.pix_x) A.pix_x[i] = px;
-      if (!(isfinite(x) && isfinite(y))) atomicOr(&g_tg_err, TG_EW_NONFINITE);
+      if (nonfinite[0]) atomicOr(&g_tg_err, TG_EW_NONFINITE);
     }
     if (A.hist) {
       bool ok = inr && (!A.mask || A.mask[i]) && py >= 0 && py < A.h && px >= 0 && px < A.w;
@@ -539,7 +528,7 @@ static int trace_fwd_impl(const tg_model* model, const tg_rays* in, tg_rays* out
   A.n = in->n;
   A.x = in->x; A.y = in->y; A.dx = in->dx; A.dy = in->dy;
   A.z = in->z; A.z_scalar = in->z_scalar;
-  A.pl = in->pathlength; A.pl_scalar = in->pl_scalar;
+  A.pl = in->pathlength; A.pl_uniform = in->pl_scalar + P.pl_const;
   A.amp = in->amplitude;
   A.ox = out->x; A.oy = out->y; A.odx = out->dx; A.ody = out->dy;
   A.opl = out->pathlength; A.oz = out->z; A.oamp = out->amplitude;
@@ -610,14 +599,22 @@ static int trace_fwd_impl(const tg_model* model, const tg_rays* in, tg_rays* out
                                      : fwd_per_sm<k_trace_fwd<4, int>>(threads))
                          : (hist_i64 ? fwd_per_sm<k_trace_fwd<1, long long>>(threads)
                                      : fwd_per_sm<k_trace_fwd<1, int>>(threads));
-  int64_t cap = (int64_t)sm_count() * per_sm;
-  int blocks = (int)(blocks_needed < cap ? blocks_needed : cap);
+  // Few rays: no more blocks than are resident, each with several turns.  From
+  // kFwdWaves waves on one turn a block, handed out as blocks finish: with
+  // fixed shares the launch waits for the SMs with the least memory bandwidth
+  // (16.8 M rays, Lens + Detector: 118 us with fixed shares, 100 with one turn
+  // a block = 0.98 of measured HBM; 2.1 M rays through five components 12.4
+  // and 13.0).
+  constexpr int64_t kFwdWaves = 8;
+  const int64_t cap = (int64_t)sm_count() * per_sm;
+  const int64_t blocks = blocks_needed <= cap || (blocks_needed >= kFwdWaves * cap && blocks_needed <= INT32_MAX)
+                             ? blocks_needed : cap;
   if (vec) {
-    if (hist_i64) k_trace_fwd<4, long long><<<blocks, threads, 0, s>>>(P, A, B);
-    else k_trace_fwd<4, int><<<blocks, threads, 0, s>>>(P, A, B);
+    if (hist_i64) k_trace_fwd<4, long long><<<(unsigned)blocks, threads, 0, s>>>(P, A, B);
+    else k_trace_fwd<4, int><<<(unsigned)blocks, threads, 0, s>>>(P, A, B);
   } else {
-    if (hist_i64) k_trace_fwd<1, long long><<<blocks, threads, 0, s>>>(P, A, B);
-    else k_trace_fwd<1, int><<<blocks, threads, 0, s>>>(P, A, B);
+    if (hist_i64) k_trace_fwd<1, long long><<<(unsigned)blocks, threads, 0, s>>>(P, A, B);
+    else k_trace_fwd<1, int><<<(unsigned)blocks, threads, 0, s>>>(P, A, B);
   }
   return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
 }
