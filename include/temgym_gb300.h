@@ -241,6 +241,8 @@ int tg_aber_monomials(const double kc[25], double w[28], double *gx, double *gy)
  *          descanner dL/d(offset x, y, dx, dy); deflector dL/d(def_x, def_y);
  *          biprism dL/d(def_x); rotator dL/d(angle in radians).
  *   workspace: device scratch of tg_trace_vjp_workspace(n) bytes.
+ * tg_trace_vjp_ex - the same for upstream gradients of which some are zero:
+ *   any array of gout may be NULL (= zero), and raw is OVERWRITTEN.
  */
 size_t tg_trace_vjp_workspace(int64_t n, const tg_model *model);
 
@@ -257,6 +259,8 @@ size_t tg_trace_adj_workspace(int64_t n, const tg_model *model);
 int tg_trace_adj(const tg_model *model, const tg_rays *in, const float *target_x,
                  const float *target_y, double *dparams, tg_rays *dray, void *workspace,
                  size_t ws_bytes, void *stream);
+int tg_trace_vjp_ex(const tg_model *model, const tg_rays *in, const tg_rays *gout,
+                    tg_rays *gin, double *raw, void *workspace, size_t ws_bytes, void *stream);
 int tg_trace_vjp(const tg_model *model, const tg_rays *in, const tg_rays *gout,
                  tg_rays *gin, double *raw, void *workspace, size_t ws_bytes,
                  void *stream);

@@ -79,6 +79,9 @@ _SIGS = {
     "tg_abcd_compose": (C.c_int, [C.POINTER(TgModel), C.POINTER(C.c_double),
                                   C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "tg_trace_vjp_workspace": (C.c_size_t, [C.c_int64, C.POINTER(TgModel)]),
+    "tg_trace_vjp_ex": (C.c_int, [C.POINTER(TgModel), C.POINTER(TgRays), C.POINTER(TgRays),
+                                  C.POINTER(TgRays), C.c_void_p, C.c_void_p, C.c_size_t,
+                                  C.c_void_p]),
     "tg_trace_vjp": (C.c_int, [C.POINTER(TgModel), C.POINTER(TgRays), C.POINTER(TgRays),
                                C.POINTER(TgRays), C.c_void_p, C.c_void_p, C.c_size_t,
                                C.c_void_p]),

@@ -79,9 +79,9 @@ __device__ __forceinline__ void sh_store_row(const uint32_t* shw, uint32_t* row,
   for (int i = threadIdx.x; i < words; i += blockDim.x) row[i] = shw[i];
 }
 
-// R consecutive floats from p + i0: 16-byte vector loads when vec (R = 4 or
-// 8, p + i0 16-byte aligned and all R in range), else per element with the
-// tail past n read as 0.  For R = 8 both vector loads are issued before the
+// R floats from p + i0: 16-byte vector loads when vec (R = 4 or 8, step 1,
+// p + i0 16-byte aligned and all R in range), else per element, step apart,
+// with the tail past n read as 0.  For R = 8 both vector loads are issued before the
 // values are unpacked (this form also spills fewer registers in the
 // 128-register adjoint).  kStream: evict-first loads (ld.global.cs), for data
 // read once by a kernel that streams many arrays.
@@ -92,7 +92,7 @@ __device__ __forceinline__ float4 ld4(const float* p) {
 
 template <int R, bool kStream = false>
 __device__ __forceinline__ void load4(const float* __restrict__ p, int64_t i0,
-                                      int64_t n, float v[R], bool vec) {
+                                      int64_t n, float v[R], bool vec, int step = 1) {
   if constexpr (R == 4) {
     if (vec) {
       const float4 t = ld4<kStream>(p + i0);
@@ -109,16 +109,14 @@ __device__ __forceinline__ void load4(const float* __restrict__ p, int64_t i0,
     }
   }
 #pragma unroll
-  for (int k = 0; k < R; ++k) v[k] = (i0 + k < n) ? __ldg(p + i0 + k) : 0.f;
+  for (int k = 0; k < R; ++k) v[k] = (i0 + k * step < n) ? __ldg(p + i0 + k * step) : 0.f;
 }
 
 // kStream: evict-first vector stores (st.global.cs).
 template <int R, bool kStream = false>
 __device__ __forceinline__ void store4(float* __restrict__ p, int64_t i0,
-                                       int64_t n, const float v[R], bool vec) {
-  if (R == 2 && vec) {
-    *reinterpret_cast<float2*>(p + i0) = make_float2(v[0], v[R - 1]);
-  } else if (R % 4 == 0 && vec) {
+                                       int64_t n, const float v[R], bool vec, int step = 1) {
+  if (R % 4 == 0 && vec) {
 #pragma unroll
     for (int q = 0; q + 3 < R; q += 4) {
       const float4 t = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
@@ -128,17 +126,17 @@ __device__ __forceinline__ void store4(float* __restrict__ p, int64_t i0,
   } else {
 #pragma unroll
     for (int k = 0; k < R; ++k)
-      if (i0 + k < n) p[i0 + k] = v[k];
+      if (i0 + k * step < n) p[i0 + k * step] = v[k];
   }
 }
 
-// The chain, the outputs, the pixels and the histogram for rays i0 .. i0+R-1
-// whose inputs are in x, y, dx, dy (vec: all R in range and every output
-// array aligned for R-wide vector stores).  All 32 lanes of the warp call it
-// (the global histogram's warp aggregation).
+// The chain, the outputs, the pixels and the histogram for rays i0 + k step,
+// k < R, whose inputs are in x, y, dx, dy (vec: step is 1, all R in range and
+// every output array aligned for R-wide vector stores).  All 32 lanes of the
+// warp call it (the global histogram's warp aggregation).
 template <int R, typename CountT, bool kSh>
 __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, const BinCoef& B,
-                                         uint32_t* shw, int64_t i0, float (&x)[R],
+                                         uint32_t* shw, int64_t i0, int step, float (&x)[R],
                                          float (&y)[R], float (&dx)[R], float (&dy)[R],
                                          bool vec) {
   const int64_t n = A.n;
@@ -159,7 +157,7 @@ __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, con
     if (A.z) {
 #pragma unroll
       for (int k = 0; k < R; ++k) {
-        dvar[k] = P.zc_first - (i0 + k < n ? A.z[i0 + k] : A.z_scalar);
+        dvar[k] = P.zc_first - (i0 + k * step < n ? A.z[i0 + k * step] : A.z_scalar);
         dvf[k] = (float)dvar[k];
       }
     }
@@ -168,10 +166,10 @@ __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, con
     for (int k = 0; k < R; ++k) {
       x[k] = r[k].x; y[k] = r[k].y; dx[k] = r[k].dx; dy[k] = r[k].dy;
     }
-    store4<R>(A.ox, i0, n, x, vec);
-    store4<R>(A.oy, i0, n, y, vec);
-    store4<R>(A.odx, i0, n, dx, vec);
-    store4<R>(A.ody, i0, n, dy, vec);
+    store4<R>(A.ox, i0, n, x, vec, step);
+    store4<R>(A.oy, i0, n, y, vec, step);
+    store4<R>(A.odx, i0, n, dx, vec, step);
+    store4<R>(A.ody, i0, n, dy, vec, step);
     if (A.opl) {
       // no float64 arithmetic per ray for a uniform base (one add per
       // per-ray input): GB300 issues float64 at ~1/64 of the float32 rate,
@@ -183,7 +181,7 @@ __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, con
       if (A.pl || A.z) {
 #pragma unroll
         for (int k = 0; k < R; ++k) {
-          double base = A.pl && i0 + k < n ? A.pl[i0 + k] + P.pl_const : A.pl_uniform;
+          double base = A.pl && i0 + k * step < n ? A.pl[i0 + k * step] + P.pl_const : A.pl_uniform;
           if (A.z) base += dvar[k];
           o[k] = add_f64_f32(base, r[k].plv);
         }
@@ -194,25 +192,23 @@ __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, con
       if (R == 4 && vec && A.opl_vec) {  // two 16-byte stores (i0 is a multiple of 4)
         reinterpret_cast<double2*>(A.opl + i0)[0] = make_double2(o[0], o[1]);
         reinterpret_cast<double2*>(A.opl + i0)[1] = make_double2(o[2 % R], o[3 % R]);
-      } else if (R == 2 && vec && A.opl_vec) {  // one 16-byte store (i0 even)
-        *reinterpret_cast<double2*>(A.opl + i0) = make_double2(o[0], o[R - 1]);
       } else {
 #pragma unroll
         for (int k = 0; k < R; ++k)
-          if (i0 + k < n) A.opl[i0 + k] = o[k];
+          if (i0 + k * step < n) A.opl[i0 + k * step] = o[k];
       }
     }
     if (A.oz) {
 #pragma unroll
       for (int k = 0; k < R; ++k)
-        if (i0 + k < n) A.oz[i0 + k] = P.z_out;
+        if (i0 + k * step < n) A.oz[i0 + k * step] = P.z_out;
     }
     if (A.oamp) {
 #pragma unroll
       for (int k = 0; k < R; ++k)
-        if (i0 + k < n) {
-          float a0 = A.amp ? A.amp[i0 + k] : 1.f;
-          A.oamp[i0 + k] = alive[k] ? a0 : 0.f;
+        if (i0 + k * step < n) {
+          float a0 = A.amp ? A.amp[i0 + k * step] : 1.f;
+          A.oamp[i0 + k * step] = alive[k] ? a0 : 0.f;
         }
     }
     if (A.do_bin) {
@@ -222,7 +218,7 @@ __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, con
 #pragma unroll
       for (int k = 0; k < R; ++k) {
         const int py = pys[k], px = pxs[k];
-        const bool inr = (i0 + k < n);
+        const bool inr = (i0 + k * step < n);
         if (inr && nonfinite[k]) atomicOr(&g_tg_err, TG_EW_NONFINITE);
         if (A.hist) {
           bool ok = inr && alive[k] && py >= 0 && py < A.h && px >= 0 && px < A.w;
@@ -231,20 +227,15 @@ __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, con
         }
       }
       // pixel indices: one vector store per array where aligned
-      if ((R == 2 || R == 4) && vec && A.pix_vec) {
-        if (R == 2) {
-          if (A.pix_y) *reinterpret_cast<int2*>(A.pix_y + i0) = make_int2(pys[0], pys[R - 1]);
-          if (A.pix_x) *reinterpret_cast<int2*>(A.pix_x + i0) = make_int2(pxs[0], pxs[R - 1]);
-        } else {
-          if (A.pix_y) *reinterpret_cast<int4*>(A.pix_y + i0) = make_int4(pys[0], pys[1 % R], pys[2 % R], pys[3 % R]);
-          if (A.pix_x) *reinterpret_cast<int4*>(A.pix_x + i0) = make_int4(pxs[0], pxs[1 % R], pxs[2 % R], pxs[3 % R]);
-        }
+      if (R == 4 && vec && A.pix_vec) {
+        if (A.pix_y) *reinterpret_cast<int4*>(A.pix_y + i0) = make_int4(pys[0], pys[1 % R], pys[2 % R], pys[3 % R]);
+        if (A.pix_x) *reinterpret_cast<int4*>(A.pix_x + i0) = make_int4(pxs[0], pxs[1 % R], pxs[2 % R], pxs[3 % R]);
       } else {
 #pragma unroll
         for (int k = 0; k < R; ++k)
-          if (i0 + k < n) {
-            if (A.pix_y) A.pix_y[i0 + k] = pys[k];
-            if (A.pix_x) A.pix_x[i0 + k] = pxs[k];
+          if (i0 + k * step < n) {
+            if (A.pix_y) A.pix_y[i0 + k * step] = pys[k];
+            if (A.pix_x) A.pix_x[i0 + k * step] = pxs[k];
           }
       }
     }
@@ -259,11 +250,19 @@ __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, con
 // 145 without prefetching).  The slots take kPfBytes ahead of the histogram words.
 constexpr int kPfBytes = 4 * kShThreads * 16;  // 64 KB
 
-template <int R, typename CountT, bool kSh = false, bool kPf = false>
+constexpr int kFwdRays = 4;  // rays a thread traces together
+
+// kVec: every array is 16-byte aligned, a thread takes R consecutive rays.
+// Else a thread's rays lie blockDim.x apart, so that each access of a warp is
+// one contiguous run whatever the arrays' alignment (an odd ray count in a
+// stacked buffer, a slice), and a step's dispatch still serves R rays:
+// 8 M rays through 8 components with pixels and image, arrays one float off:
+// 235 us with one ray a thread, 92 here, 82 aligned.
+template <int R, typename CountT, bool kVec, bool kSh = false, bool kPf = false>
 __global__ void __launch_bounds__(kSh ? kShThreads : 256)
 k_trace_fwd(const __grid_constant__ Program P, const __grid_constant__ FwdArgs A,
             const __grid_constant__ BinCoef B) {
-  static_assert(!kPf || (kSh && R == 4), "prefetch: shared-histogram variant, four rays per thread");
+  static_assert(!kPf || (kSh && kVec && R == 4), "prefetch: shared-histogram variant, four rays per thread");
   extern __shared__ __align__(16) uint32_t shm[];
   // kSh: [(h * w + 1) / 2] packed uint16 counters (after the prefetch slots with kPf)
   uint32_t* shw = kPf ? shm + kPfBytes / 4 : shm;
@@ -290,8 +289,9 @@ k_trace_fwd(const __grid_constant__ Program P, const __grid_constant__ FwdArgs A
   // block-uniform loop: every lane of every warp takes the same trip count,
   // so warp-collective histogram aggregation below is always legal.
   for (int64_t blk = (int64_t)blockIdx.x * blockDim.x * R; blk < n; blk += stride) {
-    const int64_t i0 = blk + (int64_t)threadIdx.x * R;
-    const bool vec = (R == 4) && (i0 + 3 < n);
+    const int64_t i0 = blk + (int64_t)threadIdx.x * (kVec ? R : 1);
+    const int step = kVec ? 1 : (int)blockDim.x;
+    const bool vec = kVec && (i0 + R - 1 < n);
     float x[R], y[R], dx[R], dy[R];
     if (kPf && vec) {  // the copies issued for these rays (same condition)
       cp_async_wait_all();
@@ -302,12 +302,12 @@ k_trace_fwd(const __grid_constant__ Program P, const __grid_constant__ FwdArgs A
       dx[0] = c.x; dx[1 % R] = c.y; dx[2 % R] = c.z; dx[3 % R] = c.w;
       dy[0] = d.x; dy[1 % R] = d.y; dy[2 % R] = d.z; dy[3 % R] = d.w;
     } else {
-      load4<R>(A.x, i0, n, x, vec);
-      load4<R>(A.y, i0, n, y, vec);
-      load4<R>(A.dx, i0, n, dx, vec);
-      load4<R>(A.dy, i0, n, dy, vec);
+      load4<R>(A.x, i0, n, x, vec, step);
+      load4<R>(A.y, i0, n, y, vec, step);
+      load4<R>(A.dx, i0, n, dx, vec, step);
+      load4<R>(A.dy, i0, n, dy, vec, step);
     }
-    fwd_rays<R, CountT, kSh>(P, A, B, shw, i0, x, y, dx, dy, vec);
+    fwd_rays<R, CountT, kSh>(P, A, B, shw, i0, step, x, y, dx, dy, vec);
     if (kPf) {  // the values read from the slot have been used
       if (i0 + stride + 3 < n) prefetch(i0 + stride);
       cp_async_commit();
@@ -551,36 +551,35 @@ static int trace_fwd_impl(const tg_model* model, const tg_rays* in, tg_rays* out
     // one CTA of kShThreads per SM, the detector's packed counters in shared memory
     const int bins = grid->h * grid->w;
     const size_t smem = (size_t)((bins + 1) / 2) * sizeof(uint32_t);
-    const int R = vec ? 4 : 1;
-    const int64_t need = (A.n + (int64_t)kShThreads * R - 1) / ((int64_t)kShThreads * R);
+    const int64_t per = (int64_t)kShThreads * kFwdRays, need = (A.n + per - 1) / per;
     const int blocks = (int)(need < sm_count() ? need : sm_count());
     A.rows = reinterpret_cast<uint32_t*>(workspace);
     cudaError_t e = cudaSuccess;
     if (vec && smem + kPfBytes <= (size_t)smem_optin()) {  // prefetch slots fit
       if (hist_i64) {
-        e = prefetch_attr<k_trace_fwd<4, long long, true, true>>();
+        e = prefetch_attr<k_trace_fwd<kFwdRays, long long, true, true, true>>();
         if (e == cudaSuccess)
-          k_trace_fwd<4, long long, true, true><<<blocks, kShThreads, smem + kPfBytes, s>>>(P, A, B);
+          k_trace_fwd<kFwdRays, long long, true, true, true><<<blocks, kShThreads, smem + kPfBytes, s>>>(P, A, B);
       } else {
-        e = prefetch_attr<k_trace_fwd<4, int, true, true>>();
+        e = prefetch_attr<k_trace_fwd<kFwdRays, int, true, true, true>>();
         if (e == cudaSuccess)
-          k_trace_fwd<4, int, true, true><<<blocks, kShThreads, smem + kPfBytes, s>>>(P, A, B);
+          k_trace_fwd<kFwdRays, int, true, true, true><<<blocks, kShThreads, smem + kPfBytes, s>>>(P, A, B);
       }
     } else if (vec) {
       if (hist_i64) {
-        e = shared_hist_attr<k_trace_fwd<4, long long, true>>();
-        if (e == cudaSuccess) k_trace_fwd<4, long long, true><<<blocks, kShThreads, smem, s>>>(P, A, B);
+        e = shared_hist_attr<k_trace_fwd<kFwdRays, long long, true, true>>();
+        if (e == cudaSuccess) k_trace_fwd<kFwdRays, long long, true, true><<<blocks, kShThreads, smem, s>>>(P, A, B);
       } else {
-        e = shared_hist_attr<k_trace_fwd<4, int, true>>();
-        if (e == cudaSuccess) k_trace_fwd<4, int, true><<<blocks, kShThreads, smem, s>>>(P, A, B);
+        e = shared_hist_attr<k_trace_fwd<kFwdRays, int, true, true>>();
+        if (e == cudaSuccess) k_trace_fwd<kFwdRays, int, true, true><<<blocks, kShThreads, smem, s>>>(P, A, B);
       }
     } else {
       if (hist_i64) {
-        e = shared_hist_attr<k_trace_fwd<1, long long, true>>();
-        if (e == cudaSuccess) k_trace_fwd<1, long long, true><<<blocks, kShThreads, smem, s>>>(P, A, B);
+        e = shared_hist_attr<k_trace_fwd<kFwdRays, long long, false, true>>();
+        if (e == cudaSuccess) k_trace_fwd<kFwdRays, long long, false, true><<<blocks, kShThreads, smem, s>>>(P, A, B);
       } else {
-        e = shared_hist_attr<k_trace_fwd<1, int, true>>();
-        if (e == cudaSuccess) k_trace_fwd<1, int, true><<<blocks, kShThreads, smem, s>>>(P, A, B);
+        e = shared_hist_attr<k_trace_fwd<kFwdRays, int, false, true>>();
+        if (e == cudaSuccess) k_trace_fwd<kFwdRays, int, false, true><<<blocks, kShThreads, smem, s>>>(P, A, B);
       }
     }
     if (e != cudaSuccess || cudaGetLastError() != cudaSuccess) return TG_ERR_CUDA;
@@ -590,15 +589,14 @@ static int trace_fwd_impl(const tg_model* model, const tg_rays* in, tg_rays* out
     return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
   }
   const int threads = 256;
-  const int R = vec ? 4 : 1;
-  int64_t blocks_needed = (A.n + (int64_t)threads * R - 1) / ((int64_t)threads * R);
+  const int64_t per = (int64_t)threads * kFwdRays, blocks_needed = (A.n + per - 1) / per;
   // every block resident at once: with the grid-stride loop each block has
   // the same share, so blocks waiting for a slot would lengthen the tail
   // residency per variant, queried once (a per-call query costs host time)
-  const int per_sm = vec ? (hist_i64 ? fwd_per_sm<k_trace_fwd<4, long long>>(threads)
-                                     : fwd_per_sm<k_trace_fwd<4, int>>(threads))
-                         : (hist_i64 ? fwd_per_sm<k_trace_fwd<1, long long>>(threads)
-                                     : fwd_per_sm<k_trace_fwd<1, int>>(threads));
+  const int per_sm = vec ? (hist_i64 ? fwd_per_sm<k_trace_fwd<kFwdRays, long long, true>>(threads)
+                                     : fwd_per_sm<k_trace_fwd<kFwdRays, int, true>>(threads))
+                         : (hist_i64 ? fwd_per_sm<k_trace_fwd<kFwdRays, long long, false>>(threads)
+                                     : fwd_per_sm<k_trace_fwd<kFwdRays, int, false>>(threads));
   // Few rays: no more blocks than are resident, each with several turns.  From
   // kFwdWaves waves on one turn a block, handed out as blocks finish: with
   // fixed shares the launch waits for the SMs with the least memory bandwidth
@@ -610,11 +608,11 @@ static int trace_fwd_impl(const tg_model* model, const tg_rays* in, tg_rays* out
   const int64_t blocks = blocks_needed <= cap || (blocks_needed >= kFwdWaves * cap && blocks_needed <= INT32_MAX)
                              ? blocks_needed : cap;
   if (vec) {
-    if (hist_i64) k_trace_fwd<4, long long><<<(unsigned)blocks, threads, 0, s>>>(P, A, B);
-    else k_trace_fwd<4, int><<<(unsigned)blocks, threads, 0, s>>>(P, A, B);
+    if (hist_i64) k_trace_fwd<kFwdRays, long long, true><<<(unsigned)blocks, threads, 0, s>>>(P, A, B);
+    else k_trace_fwd<kFwdRays, int, true><<<(unsigned)blocks, threads, 0, s>>>(P, A, B);
   } else {
-    if (hist_i64) k_trace_fwd<1, long long><<<(unsigned)blocks, threads, 0, s>>>(P, A, B);
-    else k_trace_fwd<1, int><<<(unsigned)blocks, threads, 0, s>>>(P, A, B);
+    if (hist_i64) k_trace_fwd<kFwdRays, long long, false><<<(unsigned)blocks, threads, 0, s>>>(P, A, B);
+    else k_trace_fwd<kFwdRays, int, false><<<(unsigned)blocks, threads, 0, s>>>(P, A, B);
   }
   return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
 }
@@ -771,7 +769,7 @@ struct VjpArgs {
   const float *x, *y, *dx, *dy;
   const double* z;
   double z_scalar;
-  const float *gx, *gy, *gdx, *gdy;
+  const float *gx, *gy, *gdx, *gdy;  // NULL: zero
   const double* gpl;
   float *ix, *iy, *idx, *idy;
   double *ipl, *iz;
@@ -784,12 +782,24 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-__device__ __forceinline__ int op_nsums(int kind) {
+__host__ __device__ __forceinline__ int op_nsums(int kind) {
   switch (kind) {
     case OP_FREE: case OP_FREE_VARZ: case OP_LENS: case OP_BIPRISM: case OP_ROTATE: case OP_ABER: return 1;
     case OP_DEFLECT: return 2;
     case OP_SHIFT: case OP_PROBE_SHIFT: return 4;
     default: return 0;
+  }
+}
+
+// load4, or zeros for an upstream gradient that is not given.
+template <int R, bool kStream = false>
+__device__ __forceinline__ void load_or_zero(const float* __restrict__ p, int64_t i0, int64_t n, float v[R],
+                                             bool vec) {
+  if (p) {
+    load4<R, kStream>(p, i0, n, v, vec);
+  } else {
+#pragma unroll
+    for (int k = 0; k < R; ++k) v[k] = 0.f;
   }
 }
 
@@ -806,7 +816,10 @@ constexpr int kVjpRays = 8;  // rays per thread on the aligned path
 // closed-form inverse, so at each one the reverse walk recomputes the state
 // entering it from the ray's input (forward steps up to the lens) and applies
 // the lens's adjoint (aber_reverse); the other steps invert as usual.
-template <int R, bool ABER>
+// kOpt: some upstream gradient is not given (NULL = zero); testing for it
+// costs the kernel registers it does not have (51 instead of 49 us for 2.1 M
+// rays through five components).
+template <int R, bool ABER, bool kOpt>
 __global__ void __launch_bounds__(kVjpThreads, 2)
 k_trace_vjp(const __grid_constant__ Program P, const __grid_constant__ VjpArgs A) {
   const float* aw = ABER ? &P.aber[0][0] : nullptr;
@@ -835,10 +848,17 @@ k_trace_vjp(const __grid_constant__ Program P, const __grid_constant__ VjpArgs A
     bool alive[R];
     float gz[R];
     float gx[R], gy[R], gdx[R], gdy[R];
-    load4<R>(A.gx, i0, n, gx, vec);
-    load4<R>(A.gy, i0, n, gy, vec);
-    load4<R>(A.gdx, i0, n, gdx, vec);
-    load4<R>(A.gdy, i0, n, gdy, vec);
+    if constexpr (kOpt) {
+      load_or_zero<R>(A.gx, i0, n, gx, vec);
+      load_or_zero<R>(A.gy, i0, n, gy, vec);
+      load_or_zero<R>(A.gdx, i0, n, gdx, vec);
+      load_or_zero<R>(A.gdy, i0, n, gdy, vec);
+    } else {
+      load4<R>(A.gx, i0, n, gx, vec);
+      load4<R>(A.gy, i0, n, gy, vec);
+      load4<R>(A.gdx, i0, n, gdx, vec);
+      load4<R>(A.gdy, i0, n, gdy, vec);
+    }
 #pragma unroll
     for (int k = 0; k < R; ++k) {
       const bool inr = i0 + k < n;
@@ -999,7 +1019,7 @@ __device__ __forceinline__ void lean_reverse(const Op& op, Ray4& r, Ray4& a, flo
       const float x = r.x, y = r.y;
       r.dx = fmaf(x, k, r.dx);
       r.dy = fmaf(y, k, r.dy);
-      c[0] = (a.dx * x + a.dy * y) * (k * k);
+      c[0] = __fmul_rn(a.dx * x + a.dy * y, k * k);  // not fused into the caller's sum, as op_reverse's is not
       a.x = a.x - a.dx * k;
       a.y = a.y - a.dy * k;
     } break;
@@ -1037,20 +1057,39 @@ __device__ __forceinline__ void lean_reverse(const Op& op, Ray4& r, Ray4& a, flo
 constexpr int kLeanRays = 8;    // rays per thread
 constexpr int kLeanBlocks = 2;  // resident blocks per SM (register bound)
 
+// One component at a time, its kind decided once for all R rays of a thread
+// (both ways: its free-space step and its own).  The sums run in the general
+// kernel's order (a thread's rays, the warp, the block's turns in float32; warps
+// and blocks in float64), so they equal its sums bit for bit.  16.8 M rays,
+// Lens + Detector: 130 us, 0.92 of measured HBM.  2.1 M rays through five
+// components with every gradient given 34.8 us (a dispatch per ray and step
+// 35.9), with those of x and y alone 31.7 (the general kernel, which gradients
+// of zeros used to take, 49.3); one block a tile, handed out by the hardware,
+// 44 and 170 us (a block's start is not hidden by two blocks an SM).
 template <int R>
 __global__ void __launch_bounds__(kVjpThreads, kLeanBlocks)
 k_trace_vjp_lean(const __grid_constant__ Program P, const __grid_constant__ VjpArgs A) {
-  __shared__ float wacc[kVjpThreads / 32][kMaxSteps * 4];
+  extern __shared__ float wacc[];  // [warps][4 n_steps] step sums
   const bool sums = A.partial != nullptr;
-  if (sums)
-    for (int i = threadIdx.x; i < (kVjpThreads / 32) * kMaxSteps * 4; i += blockDim.x) (&wacc[0][0])[i] = 0.f;
-  __syncthreads();
+  const int ns4 = 4 * P.n_steps;
+  if (sums) {
+    for (int i = threadIdx.x; i < kVjpThreads / 32 * ns4; i += kVjpThreads) wacc[i] = 0.f;
+    __syncthreads();
+  }
   const int64_t n = A.n;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x * R;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto add_sum = [&](int s, int j, float c) {
+    if (!sums) return;
+    const float v = warp_sum(c);
+    if (lane == 0) wacc[warp * ns4 + 4 * s + j] += v;
+  };
   for (int64_t blk = (int64_t)blockIdx.x * blockDim.x * R; blk < n; blk += stride) {
     const int64_t i0 = blk + (int64_t)threadIdx.x * R;
     const bool vec = i0 + R - 1 < n;
+    // short chains: the block's loads and stores in phases of their own (16.8 M
+    // rays, Lens + Detector: 135 -> 130 us)
+    if (P.n_steps <= 4) __syncthreads();
     Ray4 r[R], ad[R];
     {
       float x[R], y[R], dx[R], dy[R], gx[R], gy[R], gdx[R], gdy[R];
@@ -1058,10 +1097,10 @@ k_trace_vjp_lean(const __grid_constant__ Program P, const __grid_constant__ VjpA
       load4<R, true>(A.y, i0, n, y, vec);
       load4<R, true>(A.dx, i0, n, dx, vec);
       load4<R, true>(A.dy, i0, n, dy, vec);
-      load4<R, true>(A.gx, i0, n, gx, vec);
-      load4<R, true>(A.gy, i0, n, gy, vec);
-      load4<R, true>(A.gdx, i0, n, gdx, vec);
-      load4<R, true>(A.gdy, i0, n, gdy, vec);
+      load_or_zero<R, true>(A.gx, i0, n, gx, vec);
+      load_or_zero<R, true>(A.gy, i0, n, gy, vec);
+      load_or_zero<R, true>(A.gdx, i0, n, gdx, vec);
+      load_or_zero<R, true>(A.gdy, i0, n, gdy, vec);
 #pragma unroll
       for (int k = 0; k < R; ++k) {
         r[k] = Ray4{x[k], y[k], dx[k], dy[k]};
@@ -1069,27 +1108,44 @@ k_trace_vjp_lean(const __grid_constant__ Program P, const __grid_constant__ VjpA
         ad[k] = Ray4{gx[k], gy[k], gdx[k], gdy[k]};
       }
     }
-    for (int s = 0; s < P.n_steps; ++s) {
-      const Op op = P.op[s];
+#pragma unroll 1
+    for (int s = 0; s < P.n_steps; s += 2) {
+      auto fwd = [&](const Op& c, auto kind) {
+        Op o = c;
+        o.kind = decltype(kind)::value;
 #pragma unroll
-      for (int k = 0; k < R; ++k) lean_forward(op, r[k]);
+        for (int k = 0; k < R; ++k) lean_forward(o, r[k]);
+      };
+      if (P.op[s].kind == OP_FREE) fwd(P.op[s], OpConst<OP_FREE>());
+      const Op& c = P.op[s + 1];
+      if (c.kind == OP_LENS) fwd(c, OpConst<OP_LENS>());
+      else if (c.kind == OP_SHIFT) fwd(c, OpConst<OP_SHIFT>());
+      else if (c.kind == OP_DEFLECT) fwd(c, OpConst<OP_DEFLECT>());
+      else if (c.kind == OP_ROTATE) fwd(c, OpConst<OP_ROTATE>());
     }
-    for (int s = P.n_steps - 1; s >= 0; --s) {
-      const Op op = P.op[s];
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+    for (int s = P.n_steps - 2; s >= 0; s -= 2) {
+      auto rev = [&](int t, const Op& c, auto kind) {
+        constexpr int K = decltype(kind)::value, NS = K == OP_SHIFT ? 4 : (K == OP_DEFLECT ? 2 : 1);
+        Op o = c;
+        o.kind = K;
+        float cs[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int k = 0; k < R; ++k) {
-        float ck[4] = {0.f, 0.f, 0.f, 0.f};
-        lean_reverse(op, r[k], ad[k], ck);
-        c[0] += ck[0]; c[1] += ck[1]; c[2] += ck[2]; c[3] += ck[3];
-      }
-      if (sums) {
-        const int ns = op_nsums(op.kind);
-        for (int j = 0; j < ns; ++j) {
-          float v = warp_sum(c[j]);
-          if (lane == 0) wacc[warp][4 * s + j] += v;
+        for (int k = 0; k < R; ++k) {
+          float ck[4] = {0.f, 0.f, 0.f, 0.f};
+          lean_reverse(o, r[k], ad[k], ck);
+#pragma unroll
+          for (int j = 0; j < NS; ++j) cs[j] += ck[j];
         }
-      }
+#pragma unroll
+        for (int j = 0; j < NS; ++j) add_sum(t, j, cs[j]);
+      };
+      const Op& c = P.op[s + 1];
+      if (c.kind == OP_LENS) rev(s + 1, c, OpConst<OP_LENS>());
+      else if (c.kind == OP_SHIFT) rev(s + 1, c, OpConst<OP_SHIFT>());
+      else if (c.kind == OP_DEFLECT) rev(s + 1, c, OpConst<OP_DEFLECT>());
+      else if (c.kind == OP_ROTATE) rev(s + 1, c, OpConst<OP_ROTATE>());
+      if (P.op[s].kind == OP_FREE) rev(s, P.op[s], OpConst<OP_FREE>());
     }
     float o[R];
 #pragma unroll
@@ -1114,22 +1170,23 @@ k_trace_vjp_lean(const __grid_constant__ Program P, const __grid_constant__ VjpA
   }
   if (sums) {
     __syncthreads();
-    double* dst = A.partial + (size_t)blockIdx.x * P.n_steps * 4;
-    for (int i = threadIdx.x; i < P.n_steps * 4; i += blockDim.x) {
+    double* dst = A.partial + (size_t)blockIdx.x * ns4;
+    for (int i = threadIdx.x; i < ns4; i += kVjpThreads) {
       double t = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += (double)wacc[w][i];
+      for (int w = 0; w < kVjpThreads / 32; ++w) t += (double)wacc[w * ns4 + i];
       dst[i] = t;
     }
   }
 }
 
-// raw[i] += sum over blocks of partial[b][i]: one block per entry i, thread t
+// raw[i] += (or, with overwrite, =) the sum over blocks of partial[b][i]: one block per entry i, thread t
 // adds the blocks t, t + 256, ... in order, then a fixed shared-memory tree
 // combines the 256 sums (the same order on every run).
 constexpr int kReduceThreads = 256;
 
 __global__ void __launch_bounds__(kReduceThreads)
-k_reduce_partials(const double* __restrict__ partial, int nblocks, int width, double* __restrict__ raw) {
+k_reduce_partials(const double* __restrict__ partial, int nblocks, int width, double* __restrict__ raw,
+                  int overwrite) {
   __shared__ double sh[kReduceThreads];
   const int i = blockIdx.x;
   double a = 0.0;
@@ -1141,55 +1198,53 @@ k_reduce_partials(const double* __restrict__ partial, int nblocks, int width, do
     if (threadIdx.x < h) sh[threadIdx.x] += sh[threadIdx.x + h];
     __syncthreads();
   }
-  if (threadIdx.x == 0) raw[i] += sh[0];
+  if (threadIdx.x == 0) raw[i] = overwrite ? sh[0] : raw[i] + sh[0];
 }
 
-template <auto Kernel>
-static int vjp_per_sm() {
+// Blocks of the adjoint (either kernel: same rays a block, two blocks an SM).
+static int vjp_grid(int64_t n) {
   static int per_sm = 0;
   if (!per_sm) {
     int v = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, Kernel, kVjpThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_trace_vjp<kVjpRays, false, false>, kVjpThreads, 0);
     per_sm = v > 0 ? v : 1;
   }
-  return per_sm;
-}
-
-static int vjp_grid(int64_t n, bool lean) {
-  const int per_sm = lean ? vjp_per_sm<k_trace_vjp_lean<kLeanRays>>() : vjp_per_sm<k_trace_vjp<kVjpRays, false>>();
-  const int64_t per_block = (int64_t)kVjpThreads * (lean ? kLeanRays : kVjpRays);
-  int64_t need = (n + per_block - 1) / per_block;
-  int64_t cap = (int64_t)sm_count() * per_sm;
-  int64_t g = need < cap ? need : cap;
+  const int64_t per_block = (int64_t)kVjpThreads * kVjpRays;
+  const int64_t need = (n + per_block - 1) / per_block, cap = (int64_t)sm_count() * per_sm;
+  const int64_t g = need < cap ? need : cap;
   return (int)(g < 1 ? 1 : g);
 }
 
-// Blocks whose partial sums a workspace must hold (either kernel).
-static int vjp_grid_max(int64_t n) {
-  const int a = vjp_grid(n, false), b = vjp_grid(n, true);
-  return a > b ? a : b;
+template <int R, bool ABER>
+static void vjp_launch(const Program& P, const VjpArgs& A, int grid, bool opt, cudaStream_t s) {
+  if (opt) k_trace_vjp<R, ABER, true><<<grid, kVjpThreads, 0, s>>>(P, A);
+  else k_trace_vjp<R, ABER, false><<<grid, kVjpThreads, 0, s>>>(P, A);
 }
 
 }  // namespace tg
 
 extern "C" size_t tg_trace_vjp_workspace(int64_t n, const tg_model* model) {
   if (!model || n < 0) return 0;
-  return (size_t)vjp_grid_max(n) * (size_t)(2 * model->n_components) * 4 * sizeof(double);
+  return (size_t)vjp_grid(n) * (size_t)(2 * model->n_components) * 4 * sizeof(double);
 }
 
-extern "C" int tg_trace_vjp(const tg_model* model, const tg_rays* in, const tg_rays* gout,
-                            tg_rays* gin, double* raw, void* workspace, size_t ws_bytes,
-                            void* stream) {
+static int trace_vjp_impl(const tg_model* model, const tg_rays* in, const tg_rays* gout,
+                          tg_rays* gin, double* raw, int overwrite, void* workspace, size_t ws_bytes,
+                          void* stream) {
   if (!model || !in || !gout) return TG_ERR_INVALID;
   if (in->n < 0 || gout->n != in->n) return TG_ERR_INVALID;
-  if (in->n > 0 && (!in->x || !in->y || !in->dx || !in->dy || !gout->x || !gout->y ||
-                    !gout->dx || !gout->dy))
-    return TG_ERR_INVALID;
+  if (in->n > 0 && (!in->x || !in->y || !in->dx || !in->dy)) return TG_ERR_INVALID;
   Program P;
   int st = compile_program(model, in->z != nullptr, in->z_scalar, &P);
   if (st != TG_OK) return st;
   if (P.n_probe_ops) return TG_ERR_UNSUPPORTED;
-  if (in->n == 0) return TG_OK;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (in->n == 0) {
+    if (overwrite && raw && P.n_steps > 0 &&
+        cudaMemsetAsync(raw, 0, sizeof(double) * 4 * (size_t)P.n_steps, s) != cudaSuccess)
+      return TG_ERR_CUDA;
+    return TG_OK;
+  }
   VjpArgs A;
   std::memset(&A, 0, sizeof(A));
   A.n = in->n;
@@ -1203,28 +1258,43 @@ extern "C" int tg_trace_vjp(const tg_model* model, const tg_rays* in, const tg_r
     A.ipl = gin->pathlength; A.iz = gin->z;
   }
   A.partial = (raw && P.n_steps > 0) ? reinterpret_cast<double*>(workspace) : nullptr;
-  bool vec = al16(A.x) && al16(A.y) && al16(A.dx) && al16(A.dy) && al16(A.gx) &&
-             al16(A.gy) && al16(A.gdx) && al16(A.gdy) && (!A.ix || al16(A.ix)) &&
-             (!A.iy || al16(A.iy)) && (!A.idx || al16(A.idx)) && (!A.idy || al16(A.idy));
+  // (a NULL array is not read or written: any alignment)
+  const bool vec = al16(A.x) && al16(A.y) && al16(A.dx) && al16(A.dy) && al16(A.gx) && al16(A.gy) && al16(A.gdx) &&
+                   al16(A.gdy) && al16(A.ix) && al16(A.iy) && al16(A.idx) && al16(A.idy);
   bool lean = vec && P.n_aber == 0 && !A.z && !A.gpl;
   for (int i = 0; i < P.n_steps && lean; ++i) lean = lean_kind(P.op[i].kind);
-  const int grid = vjp_grid(in->n, lean);
+  const int grid = vjp_grid(in->n);
   const size_t need = (size_t)grid * P.n_steps * 4 * sizeof(double);
   if (A.partial && (!workspace || ws_bytes < need)) return TG_ERR_WORKSPACE;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (P.n_aber > 0) {
-    if (vec) k_trace_vjp<4, true><<<grid, kVjpThreads, 0, s>>>(P, A);
-    else k_trace_vjp<1, true><<<grid, kVjpThreads, 0, s>>>(P, A);
+  const bool opt = !A.gx || !A.gy || !A.gdx || !A.gdy;
+  if (lean) {
+    const size_t smem = sizeof(float) * (kVjpThreads / 32) * 4 * (size_t)P.n_steps;  // at most 15 KB
+    k_trace_vjp_lean<kLeanRays><<<grid, kVjpThreads, A.partial ? smem : 0, s>>>(P, A);
+  } else if (P.n_aber > 0) {
+    if (vec) vjp_launch<4, true>(P, A, grid, opt, s);
+    else vjp_launch<1, true>(P, A, grid, opt, s);
   } else {
-    if (lean) k_trace_vjp_lean<kLeanRays><<<grid, kVjpThreads, 0, s>>>(P, A);
-    else if (vec) k_trace_vjp<kVjpRays, false><<<grid, kVjpThreads, 0, s>>>(P, A);
-    else k_trace_vjp<1, false><<<grid, kVjpThreads, 0, s>>>(P, A);
+    if (vec) vjp_launch<kVjpRays, false>(P, A, grid, opt, s);
+    else vjp_launch<1, false>(P, A, grid, opt, s);
   }
   if (A.partial) {
     int width = P.n_steps * 4;
-    k_reduce_partials<<<width, kReduceThreads, 0, s>>>(A.partial, grid, width, raw);
+    k_reduce_partials<<<width, kReduceThreads, 0, s>>>(A.partial, grid, width, raw, overwrite);
   }
   return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
+}
+
+extern "C" int tg_trace_vjp(const tg_model* model, const tg_rays* in, const tg_rays* gout,
+                            tg_rays* gin, double* raw, void* workspace, size_t ws_bytes,
+                            void* stream) {
+  if (in && gout && in->n > 0 && (!gout->x || !gout->y || !gout->dx || !gout->dy)) return TG_ERR_INVALID;
+  return trace_vjp_impl(model, in, gout, gin, raw, 0, workspace, ws_bytes, stream);
+}
+
+extern "C" int tg_trace_vjp_ex(const tg_model* model, const tg_rays* in, const tg_rays* gout,
+                               tg_rays* gin, double* raw, void* workspace, size_t ws_bytes,
+                               void* stream) {
+  return trace_vjp_impl(model, in, gout, gin, raw, 1, workspace, ws_bytes, stream);
 }
 
 // ------------------------------------------------------- tg_trace_adj

@@ -30,7 +30,7 @@ import torch
 from . import _native as N
 from .components import Grid
 from .ray import GaussianRay
-from .run import _check_model, _device, pack_model
+from .run import _check_model, _device, pack_model, param_gradients
 
 FIELD_DIRECT, FIELD_SEPARABLE, FIELD_DIRECT_F64 = 0, 1, 2
 _METHODS = {"direct": FIELD_DIRECT, "separable": FIELD_SEPARABLE, "fp64": FIELD_DIRECT_F64}
@@ -307,9 +307,7 @@ class _FieldFn(torch.autograd.Function):
                 g = g.sum()
             out.append(g.to(t.dtype).reshape(t.shape))
         if spec["params"]:
-            from .run import param_gradient
-            for (i, path, t) in spec["params"]:
-                out.append(param_gradient(plan.comps, i, path, r["raw"]).to(t.dtype).reshape(t.shape))
+            out += param_gradients(plan.comps, spec["params"], r["raw"])
         return (None, *out)
 
 

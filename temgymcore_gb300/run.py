@@ -100,8 +100,11 @@ def _ray_scalar_input(ray: Ray) -> bool:
 def _fwd_launch(model, soa: _Soa, grid=None, want_pix=False, hist=None, want_amp=False, propagator=None):
     dev = soa.x.device
     n = soa.n
-    o4 = torch.empty((4, n), dtype=torch.float32, device=dev)  # one allocation, four views
-    ox, oy, odx, ody = o4[0], o4[1], o4[2], o4[3]
+    # one allocation, four views; rows padded to 16 bytes, so that every view
+    # is aligned for the kernel's vector stores whatever the ray count
+    row = (n + 3) & ~3
+    o4 = torch.empty((4, row), dtype=torch.float32, device=dev)
+    ox, oy, odx, ody = (o4[i, :n] for i in range(4))
     opl = torch.empty(n, dtype=torch.float64, device=dev)
     oamp = torch.empty(n, dtype=torch.float32, device=dev) if (want_amp or soa.amp is not None) else None
     m, keep = pack_model(model, propagator)
@@ -112,8 +115,8 @@ def _fwd_launch(model, soa: _Soa, grid=None, want_pix=False, hist=None, want_amp
     if grid is not None:
         g = grid._tg_grid()
         if want_pix:
-            pyx = torch.empty((2, n), dtype=torch.int32, device=dev)  # one allocation, two views
-            py, px = pyx[0], pyx[1]
+            pyx = torch.empty((2, row), dtype=torch.int32, device=dev)
+            py, px = pyx[0, :n], pyx[1, :n]
     if hist is not None and hist.dtype not in (torch.int32, torch.int64):
         raise TypeError("histogram accumulator must be int32 or int64")
     lib = N.lib()
@@ -161,7 +164,8 @@ def _grad_params(comps) -> list:
 
 
 def param_gradient(comps, i, path, raw):
-    """dL/d(parameter) from the adjoint's per-step sums raw[(2*n_components), 4]."""
+    """dL/d(parameter) from the adjoint's per-step sums raw[(2*n_components), 4]
+    (a float64 tensor, or a NumPy array of the sums read back to the host)."""
     c = comps[i]
     nc = len(comps)
     comp = raw[2 * i + 1]
@@ -179,22 +183,38 @@ def param_gradient(comps, i, path, raw):
     if path == "angle":
         return comp[0] * (math.pi / 180.0)
     if isinstance(c, Descanner):
-        m = torch.as_tensor(c.descan_error.as_matrix4(), dtype=torch.float64, device=raw.device)
-        s = [_f(c.scan_pos_x), _f(c.scan_pos_y), _f(c.scan_tilt_x), _f(c.scan_tilt_y)]
         g4 = comp[0:4]
-        sp = {"scan_pos_x": 0, "scan_pos_y": 1, "scan_tilt_x": 2, "scan_tilt_y": 3}
+        sp = ("scan_pos_x", "scan_pos_y", "scan_tilt_x", "scan_tilt_y")
         if path in sp:
-            j = sp[path]
+            m = c.descan_error.as_matrix4()
+            if isinstance(raw, torch.Tensor):
+                m = torch.as_tensor(m, dtype=torch.float64, device=raw.device)
+            j = sp.index(path)
             return (g4 * m[:, j]).sum() - g4[j]
         dn = path.split(".", 1)[1]
         pos = _DESCAN_POS[dn]
         if pos[0] == "off":
             return g4[pos[1]]
-        return g4[pos[0]] * s[pos[1]]
+        return g4[pos[0]] * _f(getattr(c, sp[pos[1]]))
     sp = {"scan_pos_x": 0, "scan_pos_y": 1, "scan_tilt_x": 2, "scan_tilt_y": 3}
     if path in sp:
         return comp[sp[path]]
     raise NotImplementedError(f"no gradient rule for {type(c).__name__}.{path}")
+
+
+def param_gradients(comps, plist, raw) -> list:
+    """The gradients of the parameter tensors of ``plist`` (_grad_params) from
+    the adjoint's per-step sums, each with its tensor's type and shape.
+    Host tensors take theirs from ONE readback of the sums (a copy and a wait
+    per parameter otherwise); device tensors stay on the device."""
+    host = raw.cpu().numpy() if any(not t.is_cuda for _, _, t in plist) else None
+    out = []
+    for i, path, t in plist:
+        if t.is_cuda:
+            out.append(param_gradient(comps, i, path, raw).to(t.dtype).reshape(t.shape))
+        else:
+            out.append(torch.tensor(float(param_gradient(comps, i, path, host)), dtype=t.dtype).reshape(t.shape))
+    return out
 
 
 class _TraceFn(torch.autograd.Function):
@@ -204,6 +224,7 @@ class _TraceFn(torch.autograd.Function):
         ox, oy, odx, ody, opl, zout, _, _, _ = _fwd_launch(comps, soa, propagator=spec["propagator"])
         spec["zout"] = zout
         ctx.spec = spec
+        ctx.set_materialize_grads(False)  # an output the loss does not use: no gradient to read
         return ox, oy, odx, ody, opl
 
     @staticmethod
@@ -212,38 +233,33 @@ class _TraceFn(torch.autograd.Function):
         comps, soa, plist = spec["comps"], spec["soa"], spec["params"]
         n = soa.n
         dev = soa.x.device
-        z32 = lambda: torch.zeros(n, dtype=torch.float32, device=dev)  # noqa: E731
-        gx = z32() if gx is None else gx.to(torch.float32).contiguous()
-        gy = z32() if gy is None else gy.to(torch.float32).contiguous()
-        gdx = z32() if gdx is None else gdx.to(torch.float32).contiguous()
-        gdy = z32() if gdy is None else gdy.to(torch.float32).contiguous()
+        need = ctx.needs_input_grad  # spec, x, y, dx, dy, pathlength, z, parameters
+        up = [None if g is None else g.to(torch.float32).contiguous() for g in (gx, gy, gdx, gdy)]
         gpl = None if gpl is None else gpl.to(torch.float64).contiguous()
-        ix, iy, idx, idy = z32(), z32(), z32(), z32()
-        ipl = torch.empty(n, dtype=torch.float64, device=dev)
+        gi = [torch.empty(n, dtype=torch.float32, device=dev) if need[1 + k] else None for k in range(4)]
+        ipl = None
+        if need[5]:  # d pathlength_out / d pathlength_in = 1
+            ipl = torch.zeros(n, dtype=torch.float64, device=dev) if gpl is None else \
+                torch.empty(n, dtype=torch.float64, device=dev)
         need_raw = bool(plist) or spec["z_grad"]
         m, keep = pack_model(comps, spec["propagator"])
-        raw = torch.zeros((2 * len(comps), 4), dtype=torch.float64, device=dev) if need_raw else None
+        raw = torch.empty((2 * len(comps), 4), dtype=torch.float64, device=dev) if need_raw else None
         ws = None
         if need_raw:
             nbytes = N.lib().tg_trace_vjp_workspace(n, C.byref(m))
             ws = torch.empty(max(8, nbytes), dtype=torch.uint8, device=dev)
-        gout = _rays_struct(n, gx, gy, gdx, gdy, None, 0.0, gpl, 0.0)
-        gin = _rays_struct(n, ix, iy, idx, idy, None, 0.0, ipl, 0.0)
-        st = N.lib().tg_trace_vjp(C.byref(m), C.byref(soa.struct()), C.byref(gout), C.byref(gin),
-                                  N.ptr(raw), N.ptr(ws), 0 if ws is None else ws.numel(),
-                                  N.stream_ptr())
+        gout = _rays_struct(n, *up, None, 0.0, gpl, 0.0)
+        gin = _rays_struct(n, *gi, None, 0.0, ipl if gpl is not None else None, 0.0)
+        st = N.lib().tg_trace_vjp_ex(C.byref(m), C.byref(soa.struct()), C.byref(gout), C.byref(gin),
+                                     N.ptr(raw), N.ptr(ws), 0 if ws is None else ws.numel(),
+                                     N.stream_ptr())
         del keep
-        N.check(st, "tg_trace_vjp")
-        pgrads = []
-        for (i, path, t) in plist:
-            g = param_gradient(comps, i, path, raw)
-            pgrads.append(g.to(t.dtype).reshape(t.shape))
-        gz = (-raw[0, 0]).reshape(()) if (spec["z_grad"] and raw is not None and len(comps)) else None
+        N.check(st, "tg_trace_vjp_ex")
+        pgrads = param_gradients(comps, plist, raw) if plist else []
+        gz = (-raw[0, 0]).reshape(()) if (spec["z_grad"] and len(comps)) else None
         shape = spec["shape"]
-        if gpl is None:
-            ipl = None
-        return (None, ix.reshape(shape), iy.reshape(shape), idx.reshape(shape),
-                idy.reshape(shape), ipl if ipl is None else ipl.reshape(shape), gz, *pgrads)
+        rs = lambda t: None if t is None else t.reshape(shape)  # noqa: E731
+        return (None, *(rs(t) for t in gi), rs(ipl), gz, *pgrads)
 
 
 def _needs_grad(ray, comps) -> bool:
