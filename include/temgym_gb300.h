@@ -164,12 +164,18 @@ int tg_trace_fwd(const tg_model *model, const tg_rays *in, tg_rays *out,
  * atomic per hit instead of one global atomic); otherwise the call
  * is tg_trace_fwd.  The workspace query is 0 for detectors above ~100k pixels
  * or fewer than 32 rays per pixel, where global atomics are the better choice.
+ * tg_trace_image_new - the same into a histogram that is OVERWRITTEN (zeroed
+ * on the stream first).
  */
 size_t tg_trace_image_workspace(int64_t n, const tg_grid *grid);
 int tg_trace_image(const tg_model *model, const tg_rays *in, tg_rays *out,
                    double *z_out, const tg_grid *grid, int32_t *pix_y,
                    int32_t *pix_x, void *hist, int32_t hist_i64, void *workspace,
                    size_t ws_bytes, void *stream);
+int tg_trace_image_new(const tg_model *model, const tg_rays *in, tg_rays *out,
+                       double *z_out, const tg_grid *grid, int32_t *pix_y,
+                       int32_t *pix_x, void *hist, int32_t hist_i64, void *workspace,
+                       size_t ws_bytes, void *stream);
 
 /*
  * tg_bin - metres->pixels + histogram for existing rays (no trace).

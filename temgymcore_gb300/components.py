@@ -23,8 +23,21 @@ from .tree_utils import HasParamsMixin
 
 def _f(v) -> float:
     if isinstance(v, torch.Tensor):
-        return float(v.detach().item())
+        return float(v.item())
     return float(v)
+
+
+def _plain(v) -> bool:
+    """True for values that cannot change in place: numbers, and tuples of them."""
+    return isinstance(v, (int, float, np.generic)) or v is None or (isinstance(v, tuple) and all(map(_plain, v)))
+
+
+def _frozen(obj) -> bool:
+    """True for an instance of a frozen dataclass whose fields cannot change
+    in place: what follows from them alone may be kept on the instance."""
+    params = getattr(obj, "__dataclass_params__", None)
+    return (params is not None and params.frozen
+            and all(_plain(getattr(obj, f)) for f in obj.__dataclass_fields__))
 
 
 class Component(HasParamsMixin):
@@ -49,6 +62,18 @@ class Component(HasParamsMixin):
         comp.z = _f(self.z)
         for i, v in enumerate(self._params()):
             comp.p[i] = v
+
+    def _packed(self) -> bytes:
+        """The packed TgComponent: kept on the instance while its fields are
+        plain numbers (frozen), formed anew where a field may change."""
+        b = self.__dict__.get("_packed_cache")
+        if b is None:
+            comp = N.TgComponent()
+            self._pack(comp)
+            b = bytes(comp)
+            if _frozen(self):
+                object.__setattr__(self, "_packed_cache", b)
+        return b
 
     def new_with(self, **kw):
         """tree_utils.py:168-172."""
@@ -191,6 +216,17 @@ class Grid:
             object.__setattr__(self, "_tg_grid_cache", g)
         return g
 
+    def _pixel_map(self) -> tuple:
+        """The six numbers of the pixels -> metres map (y row, then x row),
+        kept on the instance while its fields are plain numbers."""
+        t = self.__dict__.get("_pixel_map_cache")
+        if t is None:
+            m = self.pixels_to_metres_mat
+            t = tuple(float(v) for v in (m[0, 0], m[0, 1], m[0, 2], m[1, 0], m[1, 1], m[1, 2]))
+            if _frozen(self):
+                object.__setattr__(self, "_pixel_map_cache", t)
+        return t
+
     @property
     def coords_px(self):
         """grid.py:66-80."""
@@ -322,9 +358,10 @@ class Descanner(Component):
     _kind = N.DESCANNER
 
     def _params(self) -> list:
-        m = self.descan_error.as_matrix4()
-        return ([_f(self.scan_pos_x), _f(self.scan_pos_y), _f(self.scan_tilt_x),
-                 _f(self.scan_tilt_y)] + list(m.reshape(-1)) + self.descan_error.offsets())
+        e = [_f(v) for v in self.descan_error]  # p[]: scan, then as_matrix4 row by row, then the offsets
+        return [_f(self.scan_pos_x), _f(self.scan_pos_y), _f(self.scan_tilt_x), _f(self.scan_tilt_y),
+                e[0], e[1], e[12], e[13], e[2], e[3], e[14], e[15], e[4], e[5], e[16], e[17],
+                e[6], e[7], e[18], e[19], *e[8:12]]
 
 
 @dataclass(frozen=True)

@@ -637,6 +637,18 @@ extern "C" int tg_trace_image(const tg_model* model, const tg_rays* in, tg_rays*
                         ws_bytes, stream);
 }
 
+extern "C" int tg_trace_image_new(const tg_model* model, const tg_rays* in, tg_rays* out,
+                                  double* z_out, const tg_grid* grid, int32_t* pix_y,
+                                  int32_t* pix_x, void* hist, int32_t hist_i64, void* workspace,
+                                  size_t ws_bytes, void* stream) {
+  if (hist && (!grid || grid->h <= 0 || grid->w <= 0)) return TG_ERR_INVALID;
+  if (hist && cudaMemsetAsync(hist, 0, (size_t)grid->h * grid->w * (hist_i64 ? 8 : 4),
+                              reinterpret_cast<cudaStream_t>(stream)) != cudaSuccess)
+    return TG_ERR_CUDA;
+  return trace_fwd_impl(model, in, out, z_out, grid, pix_y, pix_x, hist, hist_i64, workspace,
+                        ws_bytes, stream);
+}
+
 static int bin_impl(int64_t n, const float* x, const float* y, const uint8_t* mask,
                     const tg_grid* grid, int32_t* pix_y, int32_t* pix_x, void* hist,
                     int32_t hist_i64, void* workspace, size_t ws_bytes, void* stream) {

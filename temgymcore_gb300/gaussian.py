@@ -80,6 +80,9 @@ N.register("tg_field_vjp_input_ex", C.c_int, [C.c_int32, C.POINTER(TgBeams), C.P
 
 def _f64(v, n, dev, width=None):
     if isinstance(v, torch.Tensor):
+        if (v.dtype == torch.float64 and v.device == dev and v.is_contiguous() and v.shape[0:1] == (n,)
+                and v.dim() == (1 if width is None else 2) and (width is None or v.shape[1] == width)):
+            return v.detach() if v.requires_grad else v  # already in the kernel layout
         t = v.detach().to(device=dev, dtype=torch.float64)
     else:
         t = torch.as_tensor(np.asarray(v, dtype=np.float64), device=dev)
@@ -105,11 +108,9 @@ def _upload(a: np.ndarray, dev) -> torch.Tensor:
 
 
 def pixel_map(grid: Grid) -> TgPixelMap:
-    t = grid.pixels_to_metres_mat
     pm = TgPixelMap()
     pm.h, pm.w = int(grid.shape[0]), int(grid.shape[1])
-    for i, v in enumerate((t[0, 0], t[0, 1], t[0, 2], t[1, 0], t[1, 1], t[1, 2])):
-        pm.t[i] = float(v)
+    pm.t[:] = grid._pixel_map()
     return pm
 
 
@@ -120,11 +121,15 @@ class BeamSet:
         r = rays
         n = r.size
         self.n = n
-        zs = np.unique(np.asarray(r.z.detach().cpu() if isinstance(r.z, torch.Tensor) else r.z,
-                                  dtype=np.float64).reshape(-1))
-        if zs.size > 1:
-            raise NotImplementedError("beams must start from one plane (uniform z)")
-        self.z = float(zs[0]) if zs.size else 0.0
+        if type(r.z) is float or type(r.z) is int:
+            self.z = float(r.z)
+        else:
+            zs = np.unique(np.asarray(r.z.detach().cpu() if isinstance(r.z, torch.Tensor) else r.z,
+                                      dtype=np.float64).reshape(-1))
+            if zs.size > 1:
+                raise NotImplementedError("beams must start from one plane (uniform z)")
+            self.z = float(zs[0]) if zs.size else 0.0
+        self.wl_scalar = 0.0
         a = r.amplitude
         if isinstance(a, torch.Tensor):
             at = a.detach().to(device=dev, dtype=torch.complex64).reshape(-1)
@@ -136,7 +141,17 @@ class BeamSet:
         cols = (r.x, r.y, r.dx, r.dy, r.pathlength, r.wavelength, r.theta)
         pairs = (r.waist_xy, r.radii_of_curv)
         if any(isinstance(v, torch.Tensor) for v in cols + pairs):
-            self.x, self.y, self.dx, self.dy, self.pl, self.wl, self.theta = (_f64(v, n, dev) for v in cols)
+            # one wavelength for all beams goes to the kernels as a number (no
+            # copy to the device); so does an angle of exactly 0, as no array
+            wl = theta = None
+            if isinstance(r.wavelength, (int, float)) and r.wavelength != 0:
+                self.wl_scalar = float(r.wavelength)
+            else:
+                wl = _f64(r.wavelength, n, dev)
+            if not (isinstance(r.theta, (int, float)) and r.theta == 0):
+                theta = _f64(r.theta, n, dev)
+            self.x, self.y, self.dx, self.dy, self.pl = (_f64(v, n, dev) for v in cols[:5])
+            self._wl, self._theta = wl, theta
             self.waist, self.radii = (_f64(v, n, dev, 2) for v in pairs)
             return
         # host values: packed into one float64 buffer (pinned, from the caching
@@ -153,10 +168,20 @@ class BeamSet:
             host[(7 + 2 * i) * n:(9 + 2 * i) * n] = (a2 if a2.shape[0] != 1 else
                                                      np.broadcast_to(a2, (n, 2))).reshape(-1)
         buf = staging.to(dev, non_blocking=True) if dev.type == "cuda" else staging
-        self.x, self.y, self.dx, self.dy, self.pl, self.wl, self.theta = (buf[i * n:(i + 1) * n]
-                                                                        for i in range(7))
+        self.x, self.y, self.dx, self.dy, self.pl, self._wl, self._theta = (buf[i * n:(i + 1) * n]
+                                                                          for i in range(7))
         self.waist = buf[7 * n:9 * n].view(n, 2)
         self.radii = buf[9 * n:11 * n].view(n, 2)
+
+    @property
+    def wl(self) -> torch.Tensor:
+        """Wavelength per beam."""
+        return torch.full_like(self.x, self.wl_scalar) if self._wl is None else self._wl
+
+    @property
+    def theta(self) -> torch.Tensor:
+        """Rotation per beam."""
+        return torch.zeros_like(self.x) if self._theta is None else self._theta
 
     def struct(self) -> TgBeams:
         b = TgBeams()
@@ -167,9 +192,9 @@ class BeamSet:
         b.amplitude = self.amp.data_ptr()
         b.waist_xy = self.waist.data_ptr()
         b.radii = self.radii.data_ptr()
-        b.wavelength = self.wl.data_ptr()
-        b.wavelength_scalar = 0.0
-        b.theta = self.theta.data_ptr()
+        b.wavelength = N.ptr(self._wl)
+        b.wavelength_scalar = self.wl_scalar
+        b.theta = N.ptr(self._theta)
         return b
 
 
@@ -201,7 +226,7 @@ class FieldPlan:
         off = (-self.ws.data_ptr()) % 256
         self.ws_ptr = self.ws.data_ptr() + off
         self.ws_bytes = self.ws.numel() - off
-        self.flags = torch.zeros(1, dtype=torch.int32, device=self.dev)
+        self.flags = torch.empty(1, dtype=torch.int32, device=self.dev)  # written by the preparation
         if comps is None:
             st = N.lib().tg_field_prep_input(C.byref(self.beams.struct()), C.byref(self.pm), self.ws_ptr,
                                              self.ws_bytes, self.flags.data_ptr(), N.stream_ptr())
@@ -290,7 +315,7 @@ class _FieldFn(torch.autograd.Function):
     def forward(ctx, spec, *inputs):
         plan = spec["plan"]
         ctx.spec = spec
-        return plan.evaluate(spec["method"]).clone()
+        return plan.evaluate(spec["method"])  # the plan's own buffer: nothing else evaluates it
 
     @staticmethod
     def backward(ctx, grad):
@@ -340,8 +365,7 @@ def make_gaussian_image(gaussian_rays: GaussianRay, model, batch_size: int = 128
     out = _field_autograd(gaussian_rays, model, method)
     if out is not None:
         return out
-    plan = FieldPlan(gaussian_rays, model, method)
-    return plan.evaluate().clone()
+    return FieldPlan(gaussian_rays, model, method).evaluate()
 
 
 def evaluate_gaussian_input_image(gaussian_rays: GaussianRay, grid, batch_size: int = 128,
@@ -353,8 +377,7 @@ def evaluate_gaussian_input_image(gaussian_rays: GaussianRay, grid, batch_size: 
     out = _field_autograd(gaussian_rays, None, method, grid=grid)
     if out is not None:
         return out
-    plan = FieldPlan(gaussian_rays, None, method, grid=grid)
-    return plan.evaluate().clone()
+    return FieldPlan(gaussian_rays, None, method, grid=grid).evaluate()
 
 
 def decompose_Q_inv(Q_inv, wavelength, eps: float = 1e-12):

@@ -120,6 +120,9 @@ class GaussianRay(Ray):
     def size(self) -> int:
         """Number of beams: per-beam fields have length n; waist_xy and
         radii_of_curv are (n, 2)."""
+        cached = self.__dict__.get("_size_cache")  # fields are frozen: computed once
+        if cached is not None:
+            return cached
         sizes = set()
         for f in dataclasses.fields(self):
             v = getattr(self, f.name)
@@ -131,7 +134,9 @@ class GaussianRay(Ray):
                 sizes.add(_size(v))
         sizes.discard(1) if len(sizes) > 1 else None
         assert len(sizes) <= 1, "beam fields have mismatched sizes"
-        return sizes.pop() if sizes else 1
+        n = sizes.pop() if sizes else 1
+        object.__setattr__(self, "_size_cache", n)
+        return n
 
     def derive(self, **updates):
         return dataclasses.replace(self, **{k: (v(self) if callable(v) else v)
@@ -175,6 +180,8 @@ def as_f32(v, n: int, device) -> torch.Tensor:
 
 def as_f64_or_scalar(v, n: int, device):
     """(tensor or None, scalar): per-ray float64 vector, or one uniform value."""
+    if type(v) is float or type(v) is int:
+        return None, float(v)
     if isinstance(v, torch.Tensor):
         if v.numel() == 1 and v.dim() == 0:
             return None, float(v.detach().item())

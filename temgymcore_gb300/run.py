@@ -8,14 +8,15 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import sys
 from typing import Sequence
 
 import numpy as np
 import torch
 
 from . import _native as N
-from .components import Component, Descanner, Grid, ThickLens, Source, _f
-from .propagator import FreeSpaceParaxial, Propagator
+from .components import Component, DescanError, Descanner, Grid, ThickLens, Source, _f
+from .propagator import FreeSpaceDirCosine, FreeSpaceParaxial, Propagator
 from .ray import Ray, as_f32, as_f64_or_scalar
 
 
@@ -35,7 +36,6 @@ def _check_model(model) -> list:
 
 def _prop_code(propagator) -> int:
     """C-ABI propagator selector (TG_PROP_*) of a propagator object."""
-    from .propagator import FreeSpaceDirCosine
     if propagator is None or isinstance(propagator, FreeSpaceParaxial):
         return N.PROP_PARAXIAL
     if isinstance(propagator, FreeSpaceDirCosine):
@@ -43,13 +43,17 @@ def _prop_code(propagator) -> int:
     raise NotImplementedError(f"{type(propagator).__name__} is not a GPU propagator")
 
 
+def pack_components(comps):
+    """The component table of a checked model (ctypes array, at least one entry)."""
+    arr = (N.TgComponent * max(1, len(comps)))
+    return arr.from_buffer_copy(b"".join([c._packed() for c in comps])) if comps else arr()
+
+
 def pack_model(model, propagator=None):
     """(TgModel, keep-alive array) for a sequence of components; ``propagator``
     selects the free-space model between them (default paraxial)."""
     comps = _check_model(model)
-    arr = (N.TgComponent * max(1, len(comps)))()
-    for i, c in enumerate(comps):
-        c._pack(arr[i])
+    arr = pack_components(comps)
     m = N.TgModel()
     m.n_components = len(comps)
     m.propagator = _prop_code(propagator)
@@ -81,7 +85,7 @@ class _Soa:
         self.dy = as_f32(ray.dy, n, device)
         self.z_t, self.z_s = as_f64_or_scalar(ray.z, n, device)
         self.pl_t, self.pl_s = as_f64_or_scalar(ray.pathlength, n, device)
-        amp = getattr(ray, "amplitude", None)
+        amp = None if type(ray) is Ray else getattr(ray, "amplitude", None)
         self.amp = None
         if amp is not None and not isinstance(amp, complex) and not np.iscomplexobj(np.asarray(
                 amp.detach().cpu() if isinstance(amp, torch.Tensor) else amp)):
@@ -97,17 +101,22 @@ def _ray_scalar_input(ray: Ray) -> bool:
                getattr(ray, f).ndim == 0 for f in ("x", "y", "dx", "dy"))
 
 
-def _fwd_launch(model, soa: _Soa, grid=None, want_pix=False, hist=None, want_amp=False, propagator=None):
+def _rows(k, n, dtype, dev):
+    """k vectors of n elements in one allocation, each row padded to 16 bytes
+    (4-byte types), so that all of them are aligned for the kernels' vector
+    accesses whatever n is."""
+    t = torch.empty_strided((k, n), ((n + 3) & ~3, 1), dtype=dtype, device=dev)
+    return [t[i] for i in range(k)]
+
+
+def _fwd_launch(model, soa: _Soa, grid=None, want_pix=False, hist=None, want_amp=False, propagator=None,
+                zero_hist=False, packed=None):
     dev = soa.x.device
     n = soa.n
-    # one allocation, four views; rows padded to 16 bytes, so that every view
-    # is aligned for the kernel's vector stores whatever the ray count
-    row = (n + 3) & ~3
-    o4 = torch.empty((4, row), dtype=torch.float32, device=dev)
-    ox, oy, odx, ody = (o4[i, :n] for i in range(4))
+    ox, oy, odx, ody = _rows(4, n, torch.float32, dev)
     opl = torch.empty(n, dtype=torch.float64, device=dev)
     oamp = torch.empty(n, dtype=torch.float32, device=dev) if (want_amp or soa.amp is not None) else None
-    m, keep = pack_model(model, propagator)
+    m, keep = pack_model(model, propagator) if packed is None else packed
     out = _rays_struct(n, ox, oy, odx, ody, None, 0.0, opl, 0.0, oamp)
     zout = C.c_double(0.0)
     py = px = None
@@ -115,18 +124,18 @@ def _fwd_launch(model, soa: _Soa, grid=None, want_pix=False, hist=None, want_amp
     if grid is not None:
         g = grid._tg_grid()
         if want_pix:
-            pyx = torch.empty((2, row), dtype=torch.int32, device=dev)
-            py, px = pyx[0, :n], pyx[1, :n]
+            py, px = _rows(2, n, torch.int32, dev)
     if hist is not None and hist.dtype not in (torch.int32, torch.int64):
         raise TypeError("histogram accumulator must be int32 or int64")
     lib = N.lib()
     # many rays per pixel: per-SM shared-memory histograms summed at the end
     ws_bytes = lib.tg_trace_image_workspace(n, C.byref(g)) if (hist is not None and g is not None) else 0
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev) if ws_bytes else None
-    st = lib.tg_trace_image(C.byref(m), C.byref(soa.struct()), C.byref(out), C.byref(zout),
-                            C.byref(g) if g is not None else None, N.ptr(py), N.ptr(px),
-                            N.ptr(hist), 1 if (hist is not None and hist.dtype == torch.int64) else 0,
-                            N.ptr(ws), ws_bytes, N.stream_ptr())
+    fn = lib.tg_trace_image_new if zero_hist else lib.tg_trace_image
+    st = fn(C.byref(m), C.byref(soa.struct()), C.byref(out), C.byref(zout),
+            C.byref(g) if g is not None else None, N.ptr(py), N.ptr(px),
+            N.ptr(hist), 1 if (hist is not None and hist.dtype == torch.int64) else 0,
+            N.ptr(ws), ws_bytes, N.stream_ptr())
     del keep
     N.check(st, "tg_trace_image")
     return ox, oy, odx, ody, opl, zout.value, oamp, py, px
@@ -150,12 +159,16 @@ def _grad_params(comps) -> list:
     """(component index, path, tensor) for every parameter tensor needing grad."""
     out = []
     for i, c in enumerate(comps):
+        if not any(isinstance(v, (torch.Tensor, DescanError)) for v in c.__dict__.values()):
+            continue
         names = [f for f in getattr(c, "__dataclass_fields__", {})]
         for name in names:
             v = getattr(c, name)
             if isinstance(v, torch.Tensor) and v.requires_grad:
                 out.append((i, name, v))
             if name == "descan_error":
+                if not any(isinstance(e, torch.Tensor) for e in v):
+                    continue
                 for dn in _DESCAN_FIELDS:
                     dv = getattr(v, dn)
                     if isinstance(dv, torch.Tensor) and dv.requires_grad:
@@ -213,7 +226,8 @@ def param_gradients(comps, plist, raw) -> list:
         if t.is_cuda:
             out.append(param_gradient(comps, i, path, raw).to(t.dtype).reshape(t.shape))
         else:
-            out.append(torch.tensor(float(param_gradient(comps, i, path, host)), dtype=t.dtype).reshape(t.shape))
+            g = torch.tensor(float(param_gradient(comps, i, path, host)), dtype=t.dtype)
+            out.append(g if t.dim() == 0 else g.reshape(t.shape))
     return out
 
 
@@ -221,7 +235,8 @@ class _TraceFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, spec, x, y, dx, dy, pl, zin, *params):
         comps, soa = spec["comps"], spec["soa"]
-        ox, oy, odx, ody, opl, zout, _, _, _ = _fwd_launch(comps, soa, propagator=spec["propagator"])
+        spec["packed"] = pack_model(comps, spec["propagator"])  # the parameters' values, for both passes
+        ox, oy, odx, ody, opl, zout, _, _, _ = _fwd_launch(comps, soa, packed=spec["packed"])
         spec["zout"] = zout
         ctx.spec = spec
         ctx.set_materialize_grads(False)  # an output the loss does not use: no gradient to read
@@ -242,7 +257,7 @@ class _TraceFn(torch.autograd.Function):
             ipl = torch.zeros(n, dtype=torch.float64, device=dev) if gpl is None else \
                 torch.empty(n, dtype=torch.float64, device=dev)
         need_raw = bool(plist) or spec["z_grad"]
-        m, keep = pack_model(comps, spec["propagator"])
+        m = spec["packed"][0]
         raw = torch.empty((2 * len(comps), 4), dtype=torch.float64, device=dev) if need_raw else None
         ws = None
         if need_raw:
@@ -253,7 +268,6 @@ class _TraceFn(torch.autograd.Function):
         st = N.lib().tg_trace_vjp_ex(C.byref(m), C.byref(soa.struct()), C.byref(gout), C.byref(gin),
                                      N.ptr(raw), N.ptr(ws), 0 if ws is None else ws.numel(),
                                      N.stream_ptr())
-        del keep
         N.check(st, "tg_trace_vjp_ex")
         pgrads = param_gradients(comps, plist, raw) if plist else []
         gz = (-raw[0, 0]).reshape(()) if (spec["z_grad"] and len(comps)) else None
@@ -262,14 +276,10 @@ class _TraceFn(torch.autograd.Function):
         return (None, *(rs(t) for t in gi), rs(ipl), gz, *pgrads)
 
 
-def _needs_grad(ray, comps) -> bool:
-    if not torch.is_grad_enabled():
-        return False
-    for f in ("x", "y", "dx", "dy", "pathlength", "z"):
-        v = getattr(ray, f)
-        if isinstance(v, torch.Tensor) and v.requires_grad:
-            return True
-    return bool(_grad_params(comps))
+def _needs_grad(ray, plist) -> bool:
+    """A ray field or a parameter (plist: _grad_params) requires grad."""
+    return bool(plist) or any(isinstance(v, torch.Tensor) and v.requires_grad
+                              for v in (ray.x, ray.y, ray.dx, ray.dy, ray.pathlength, ray.z))
 
 
 def _in_shape(ray: Ray):
@@ -292,18 +302,14 @@ def run_to_end(ray: Ray, components: Sequence[Component],
     dev = _device()
     soa = _Soa(ray, dev)
     shape = _in_shape(ray)
-    if _needs_grad(ray, comps):
-        plist = _grad_params(comps)
+    plist = _grad_params(comps) if torch.is_grad_enabled() else []
+    if torch.is_grad_enabled() and _needs_grad(ray, plist):
         zt = ray.z if isinstance(ray.z, torch.Tensor) and ray.z.requires_grad and ray.z.dim() == 0 else None
         spec = {"comps": comps, "soa": soa, "params": plist, "shape": shape,
                 "z_grad": zt is not None, "propagator": propagator}
-        xs = [ray.x, ray.y, ray.dx, ray.dy]
-        xs = [v if isinstance(v, torch.Tensor) and v.requires_grad else
-              torch.zeros((), device=dev) for v in xs]
-        pl = ray.pathlength if isinstance(ray.pathlength, torch.Tensor) and ray.pathlength.requires_grad \
-            else torch.zeros((), device=dev, dtype=torch.float64)
-        zin = zt if zt is not None else torch.zeros((), device=dev, dtype=torch.float64)
-        ox, oy, odx, ody, opl = _TraceFn.apply(spec, *xs, pl, zin, *[p[2] for p in plist])
+        xs = [v if isinstance(v, torch.Tensor) and v.requires_grad else None
+              for v in (ray.x, ray.y, ray.dx, ray.dy, ray.pathlength)]
+        ox, oy, odx, ody, opl = _TraceFn.apply(spec, *xs, zt, *[p[2] for p in plist])
         zout = spec["zout"]
     else:
         ox, oy, odx, ody, opl, zout, _, _, _ = _fwd_launch(comps, soa, propagator=propagator)
@@ -725,15 +731,21 @@ def trace_to_image(ray: Ray, components: Sequence[Component], detector: Grid | N
     dev = _device()
     soa = _Soa(ray, dev)
     h, w = int(detector.shape[0]), int(detector.shape[1])
-    if acc is None:
-        acc = torch.zeros((h, w), dtype=torch.int64, device=dev)
-    ox, oy, odx, ody, opl, zout, oamp, py, px = _fwd_launch(comps, soa, detector, want_pixels, acc)
+    new = acc is None
+    if new:
+        acc = torch.empty((h, w), dtype=torch.int64, device=dev)  # zeroed by the call
+    ox, oy, odx, ody, opl, zout, oamp, py, px = _fwd_launch(comps, soa, detector, want_pixels, acc,
+                                                            zero_hist=new)
     shape = _in_shape(ray)
     rs = _reshaper(shape, soa.n)
     out = Ray(x=rs(ox), y=rs(oy), dx=rs(odx), dy=rs(ody), z=zout, pathlength=rs(opl), _one=ray._one)
-    from . import PixelsYX
-    pix = PixelsYX(y=rs(py), x=rs(px)) if want_pixels else None
+    pix = _pixels_yx()(y=rs(py), x=rs(px)) if want_pixels else None
     return out, pix, acc
+
+
+def _pixels_yx():
+    """The package's PixelsYX (defined by the package module, which imports this one)."""
+    return sys.modules[__package__].PixelsYX
 
 
 def _reshaper(shape, n):

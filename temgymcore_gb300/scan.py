@@ -18,7 +18,7 @@ import torch
 from . import _native as N
 from .components import Descanner, Detector, Grid, ScanGrid, Scanner
 from .ray import Ray, as_f32, as_f64_or_scalar
-from .run import _check_model, _device, _rays_struct
+from .run import _check_model, _device, _rays_struct, pack_components
 
 N.register("tg_scan_hist", C.c_int, [C.POINTER(N.TgModel), C.POINTER(N.TgRays), C.c_void_p,
                                      C.POINTER(N.TgGrid), C.c_void_p, C.c_void_p, C.c_void_p])
@@ -31,9 +31,8 @@ class TgScan(C.Structure):
 
 def pack_scan_model(model):
     comps = _check_model(model)
-    arr = (N.TgComponent * max(1, len(comps)))()
+    arr = pack_components(comps)
     for i, c in enumerate(comps):
-        c._pack(arr[i])
         if isinstance(c, (Scanner, Descanner)):
             arr[i].flags = N.FLAG_PER_PROBE
     m = N.TgModel()
@@ -52,11 +51,9 @@ def scan_struct(scan_grid: ScanGrid | None, positions=None, n_probes=None):
         s.positions = pos.data_ptr()
         keep = pos
     else:
-        t = scan_grid.pixels_to_metres_mat
         s.n_probes = int(scan_grid.shape[0]) * int(scan_grid.shape[1]) if n_probes is None else n_probes
         s.cols = int(scan_grid.shape[1])
-        for i, v in enumerate((t[0, 0], t[0, 1], t[0, 2], t[1, 0], t[1, 1], t[1, 2])):
-            s.t[i] = float(v)
+        s.t[:] = scan_grid._pixel_map()
         s.positions = None
     return s, keep
 
