@@ -9,9 +9,10 @@
 //   k_field_direct<L>   fast direct sum (any Q2, the astigmatic case): each
 //                       thread owns a strip of L pixels of one row; per beam it
 //                       evaluates the exact fixed-point phase and the envelope
-//                       at the strip start, then walks the strip with two
-//                       complex multiplications per pixel (a geometric
-//                       recurrence: the phase/envelope are quadratic in col).
+//                       at the strip start, then walks the strip two pixels at
+//                       a time: a running linear factor times the beam's own
+//                       quadratic factor, tabulated once per block (the
+//                       phase/envelope are quadratic in col).
 //   k_field_direct_f64  the all-float64 comparator: evaluates the polynomial,
 //                       sin/cos and exp in float64 for every (beam, pixel).
 //   k_field_operands    separable case: per-beam row and column phasor
@@ -324,7 +325,7 @@ k_field_prep(const __grid_constant__ DModel M, const __grid_constant__ PrepArgs 
 
 // ---------------------------------------------------------------- direct
 constexpr int kDirThreads = 256;
-constexpr int kBeamBatch = 64;
+constexpr int kBeamBatch = 128;
 
 struct DirArgs {
   const BeamFast* beams;
@@ -337,37 +338,75 @@ struct DirArgs {
 };
 
 // Per (beam, strip) the log-amplitude decides how the strip is summed: skip
-// when it stays below kDirSkipLog (e^-60 of a unit amplitude), the geometric
-// recurrence while its start and per-step ratios stay inside float32 range
-// (|log| < 80), otherwise a per-pixel evaluation.
+// when it stays below kDirSkipLog (e^-60 of a unit amplitude); with the beam's
+// ratio table while the strip's linear part stays inside float32 range (|log| <
+// kDirRecurMax); else the geometric recurrence while its start and per-step
+// ratios do; otherwise a per-pixel evaluation.
 constexpr float kDirSkipLog = -60.f;
 constexpr float kDirRecurMax = 80.f;
-// Strips of 32 pixels with the recurrence restarted exactly after 16: the
-// per-(beam, strip) set-up (exact phase, envelope range) is paid once per 32
-// pixels and the float32 recurrence error stays that of 16 steps.  Measured
-// at 16,384 beams, 512^2: 16-pixel strips 2.25 ms (4.5e-6 of the float64
-// kernel), 32 without restart 1.81 ms (1.2e-5), 32 with restart 2.01 ms
-// (4.0e-6), 24 pixels 2.46 ms.
-constexpr int kDirRestart = 16;  // pixels between exact restarts of the recurrence
+constexpr int kDirRestart = 16;  // pixels between exact restarts
+
+// Packed float32 pairs (two pixels of a strip): one issue slot for two
+// multiply-adds.
+__device__ __forceinline__ uint64_t pk(float lo, float hi) {
+  return (uint64_t)__float_as_uint(lo) | ((uint64_t)__float_as_uint(hi) << 32);
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ void add_lo(uint64_t& a, float v) {
+  a = (a & 0xffffffff00000000ull) | __float_as_uint(__uint_as_float((uint32_t)a) + v);
+}
+__device__ __forceinline__ void add_hi(uint64_t& a, float v) {
+  a = (a & 0xffffffffull) | ((uint64_t)__float_as_uint(__uint_as_float((uint32_t)(a >> 32)) + v) << 32);
+}
+
+// A beam's value at column j of a strip is z w^j R_j: z and w belong to the
+// strip (value and linear step at its start), R_j = rho^(j (j - 1) / 2) to the
+// beam alone.  The block forms R once per beam (256 strips use it), pixel pairs
+// as packed floats: {Re, Im, -Im}.  Bound by the FMA pipe (a packed multiply-add
+// takes it for two cycles: 8 per pixel) and the set-up of a strip (~70
+// instructions).  Measured at 16,384 astigmatic beams on 512^2 (1.8e-6 of the
+// 64-bit field): 1.38 ms; with both factors as recurrences, an anchor every 16
+// pixels and four rows of eight strips a warp 1.85 ms (1.9e-6); the table over 16
+// pixels and an anchor between 1.55 (1.2e-6); 64 instead of 128 beams a batch 1.40
+// (barriers); 64 or 128 rows a tile 1.41 / 1.39, and 52 -> 55 us at 300 beams.
+struct alignas(16) Ratio2 {
+  uint64_t re, im;
+  uint64_t nim, pad;
+};
 
 template <int L>
-__global__ void __launch_bounds__(kDirThreads)
+__global__ void __launch_bounds__(kDirThreads, 2)
 k_field_direct(const __grid_constant__ DirArgs A) {
-  __shared__ BeamFast sb[kBeamBatch];
+  static_assert(L % kDirRestart == 0 && kDirRestart % 2 == 0, "whole pixel pairs between restarts");
+  constexpr int H = L / 2;
+  extern __shared__ __align__(16) unsigned char dir_smem[];  // the batch's records, then its ratio tables
+  BeamFast* sb = reinterpret_cast<BeamFast*>(dir_smem);
+  Ratio2 (*tab)[H] = reinterpret_cast<Ratio2 (*)[H]>(dir_smem + kBeamBatch * sizeof(BeamFast));
   const int tiles_x = (A.w + A.strips_x * L - 1) / (A.strips_x * L);
   const int tx = blockIdx.x % tiles_x, ty = blockIdx.x / tiles_x;
-  const int lr = threadIdx.x / A.strips_x, ls = threadIdx.x % A.strips_x;
+  // a warp is one strip column of the tile's 32 rows: a compact patch, so its
+  // lanes agree on what is far enough to skip (24 of 32 lanes were active with
+  // four rows of the tile's eight strips a warp)
+  const int warp = threadIdx.x >> 5;
+  const int lr = (threadIdx.x & 31) + 32 * (warp / A.strips_x), ls = warp % A.strips_x;
   const int row = ty * A.tile_rows + lr;
   const int col0 = (tx * A.strips_x + ls) * L;
   const int64_t b0 = (int64_t)blockIdx.y * A.chunk;
   int64_t b1 = b0 + A.chunk;
   if (b1 > A.n) b1 = A.n;
-  float are[L], aim[L];
+  uint64_t ar[H], ai[H];  // pixel pairs of the strip
 #pragma unroll
-  for (int j = 0; j < L; ++j) { are[j] = 0.f; aim[j] = 0.f; }
-  const uint64_t urow = (uint64_t)row, ucol = (uint64_t)col0;
-  const uint64_t urow2 = urow * urow, ucol2 = ucol * ucol, urc = urow * ucol;
-  const uint64_t ustep = 2 * ucol + 1;
+  for (int j = 0; j < H; ++j) ar[j] = ai[j] = 0ull;
+  const uint32_t urow = (uint32_t)row, ucol = (uint32_t)col0;
   for (int64_t bb = b0; bb < b1; bb += kBeamBatch) {
     const int nb = (int)((b1 - bb) < kBeamBatch ? (b1 - bb) : kBeamBatch);
     __syncthreads();
@@ -378,54 +417,78 @@ k_field_direct(const __grid_constant__ DirArgs A) {
       for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
     }
     __syncthreads();
+    for (int i = threadIdx.x; i < nb * H; i += blockDim.x) {
+      const int k = i / H, j = 2 * (i % H);
+      const BeamFast& B = sb[k];
+      const float f0 = (float)(j * (j - 1)), f1 = (float)((j + 1) * j);
+      const float2 r0 = cexpf_turn(-B.b_cc * f0, B.p_cc * (uint64_t)(int64_t)(j * (j - 1)));
+      const float2 r1 = cexpf_turn(-B.b_cc * f1, B.p_cc * (uint64_t)((j + 1) * j));
+      tab[k][j / 2] = Ratio2{pk(r0.x, r1.x), pk(r0.y, r1.y), pk(-r0.y, -r1.y), 0ull};
+    }
+    __syncthreads();
     for (int k = 0; k < nb; ++k) {
       const BeamFast& B = sb[k];
-      // exact phase at the strip start and its first column step
-      uint64_t th = B.p_cc * ucol2 + B.p_rr * urow2 + B.p_rc * urc + B.p_c * ucol + B.p_r * urow + B.p_0;
-      uint64_t dth = B.p_cc * ustep + B.p_rc * urow + B.p_c;
+      // exact phase at the strip start and its first column step (Horner, so
+      // that every factor beside a 64-bit coefficient has 32 bits)
+      const uint64_t lin = B.p_cc * ucol + B.p_rc * urow + B.p_c;
+      uint64_t th = lin * ucol + ((B.p_rr * urow + B.p_r) * urow + B.p_0);
+      uint64_t dth = lin + B.p_cc * (ucol + 1u);
       const float dr = (float)row - B.r0, dc = (float)col0 - B.c0;
-      const float la = B.e0 - (B.b_cc * dc * dc + B.b_rr * dr * dr + B.b_rc * dr * dc + B.l_c * dc + B.l_r * dr);
-      const float dla = -(B.b_cc * (2.f * dc + 1.f) + B.b_rc * dr + B.l_c);
-      // log-amplitude along the strip: la(j) = la + j dla - b_cc j (j - 1)
+      // the log-amplitude and its column step at offset d from the centre,
+      // evaluated directly where values are formed: summing la + j dla -
+      // b_cc j (j - 1) over a strip cancels terms of a few hundred down to the
+      // value and costs float32 accuracy
+      const float rowlog = B.e0 - dr * fmaf(B.b_rr, dr, B.l_r), slope = fmaf(B.b_rc, dr, B.l_c);
+      auto la_at = [&](float d) { return fmaf(-d, fmaf(B.b_cc, d, slope), rowlog); };
+      auto dla_at = [&](float d) { return -fmaf(B.b_cc, 2.f * d + 1.f, slope); };
+      const float la = la_at(dc), dla = dla_at(dc);
+      // log-amplitude along the strip: la(j) = la + j dla - b_cc j (j - 1); its
+      // largest value at the ends or at the vertex j = 1/2 + dla / (2 b_cc)
       const float jl = (float)(L - 1);
       const float la_end = la + jl * dla - B.b_cc * jl * (jl - 1.f);
       const float dla_end = dla - 2.f * B.b_cc * (jl - 1.f);
-      float jv = B.b_cc > 0.f ? 0.5f + dla / (2.f * B.b_cc) : (dla > 0.f ? jl : 0.f);
+      float jv = B.b_cc > 0.f ? 0.5f + __fdividef(dla, 2.f * B.b_cc) : (dla > 0.f ? jl : 0.f);
       jv = fminf(fmaxf(jv, 0.f), jl);
       const float la_max = fmaxf(fmaxf(la, la_end), la + jv * dla - B.b_cc * jv * (jv - 1.f));
       if (!(la_max > kDirSkipLog)) continue;  // below e^-60 of unit amplitude everywhere (or NaN)
-      // the log-amplitude and its column step at offset d from the centre,
-      // evaluated directly (as la itself) where values are formed: summing
-      // la + j dla - b_cc j (j - 1) over a 32-pixel strip cancels terms of a
-      // few hundred down to the value and costs float32 accuracy
-      auto la_at = [&](float d) {
-        return B.e0 - (B.b_cc * d * d + B.b_rr * dr * dr + B.b_rc * dr * d + B.l_c * d + B.l_r * dr);
-      };
-      auto dla_at = [&](float d) { return -(B.b_cc * (2.f * d + 1.f) + B.b_rc * dr + B.l_c); };
-      if (la > -kDirRecurMax && fabsf(dla) < kDirRecurMax && fabsf(dla_end) < kDirRecurMax) {
-        // the geometric recurrence stays inside float32 range: z_j+1 = z_j w_j, w_j+1 = w_j rho
+      // the exponents that the ratio table splits apart, R_j and z w^j (below
+      // e^-80 the pixel's own value is smaller still)
+      const float dmax = fmaxf(fabsf(dla), fabsf(dla_end));
+      if (fabsf(B.b_cc) * (jl * (jl - 1.f)) < kDirRecurMax && la > -kDirRecurMax && la_max + jl * dmax < kDirRecurMax) {
+        const float2 z0 = cexpf_turn(la, th), z1 = cexpf_turn(la + dla, th + dth), w = cexpf_turn(2.f * dla, 2 * dth);
+        uint64_t zr = pk(z0.x, z1.x), zi = pk(z0.y, z1.y);
+        const uint64_t wr = pk(w.x, w.x), wi = pk(w.y, w.y), nwi = pk(-w.y, -w.y);
+#pragma unroll
+        for (int j = 0; j < H; ++j) {
+          const uint64_t rr = tab[k][j].re, ri = tab[k][j].im, nri = tab[k][j].nim;
+          ar[j] = fma2(zr, rr, ar[j]);
+          ai[j] = fma2(zr, ri, ai[j]);
+          ar[j] = fma2(zi, nri, ar[j]);
+          ai[j] = fma2(zi, rr, ai[j]);
+          if (j + 1 < H) {
+            const uint64_t t = mul2(zr, wr), u = mul2(zr, wi);
+            zr = fma2(zi, nwi, t);
+            zi = fma2(zi, wr, u);
+          }
+        }
+      } else if (la > -kDirRecurMax && fabsf(dla) < kDirRecurMax && fabsf(dla_end) < kDirRecurMax) {
+        // the geometric recurrence stays inside float32 range: z_j+1 = z_j w_j,
+        // w_j+1 = w_j rho, re-anchored at the exact value every kDirRestart pixels
         float2 z = cexpf_turn(la, th);
         float2 w = cexpf_turn(dla, dth);
         const float rr = B.rho_re, ri = B.rho_im;
 #pragma unroll
         for (int j = 0; j < L; ++j) {
           if (j > 0 && j % kDirRestart == 0) {
-            // re-anchor every kDirRestart pixels at the exact value (the
-            // phase at column j by integer differences), so the float32
-            // recurrence error stays that of kDirRestart steps
             const float dj = dc + (float)j;
             const uint64_t uj = (uint64_t)j;
             z = cexpf_turn(la_at(dj), th + uj * dth + uj * (uj - 1) * B.p_cc);
             w = cexpf_turn(dla_at(dj), dth + 2 * uj * B.p_cc);
           }
-          are[j] += z.x;
-          aim[j] += z.y;
-          float zr = z.x * w.x - z.y * w.y;
-          float zi = z.x * w.y + z.y * w.x;
-          z = make_float2(zr, zi);
-          float wr = w.x * rr - w.y * ri;
-          float wi = w.x * ri + w.y * rr;
-          w = make_float2(wr, wi);
+          if (j & 1) { add_hi(ar[j / 2], z.x); add_hi(ai[j / 2], z.y); }
+          else { add_lo(ar[j / 2], z.x); add_lo(ai[j / 2], z.y); }
+          z = make_float2(z.x * w.x - z.y * w.y, z.x * w.y + z.y * w.x);
+          w = make_float2(w.x * rr - w.y * ri, w.x * ri + w.y * rr);
         }
       } else {
         // a beam narrow against the strip: every pixel evaluated directly
@@ -434,8 +497,8 @@ k_field_direct(const __grid_constant__ DirArgs A) {
 #pragma unroll
         for (int j = 0; j < L; ++j) {
           const float2 z = cexpf_turn(la_at(dc + (float)j), th);
-          are[j] += z.x;
-          aim[j] += z.y;
+          if (j & 1) { add_hi(ar[j / 2], z.x); add_hi(ai[j / 2], z.y); }
+          else { add_lo(ar[j / 2], z.x); add_lo(ai[j / 2], z.y); }
           th += dth;
           dth += ddth;
         }
@@ -445,8 +508,12 @@ k_field_direct(const __grid_constant__ DirArgs A) {
   if (row < A.h) {
     float2* o = A.out + (size_t)blockIdx.y * A.h * A.w + (size_t)row * A.w;
 #pragma unroll
-    for (int j = 0; j < L; ++j)
-      if (col0 + j < A.w) o[col0 + j] = make_float2(are[j], aim[j]);
+    for (int j = 0; j < H; ++j) {
+      if (col0 + 2 * j < A.w)
+        o[col0 + 2 * j] = make_float2(__uint_as_float((uint32_t)ar[j]), __uint_as_float((uint32_t)ai[j]));
+      if (col0 + 2 * j + 1 < A.w)
+        o[col0 + 2 * j + 1] = make_float2(__uint_as_float((uint32_t)(ar[j] >> 32)), __uint_as_float((uint32_t)(ai[j] >> 32)));
+    }
   }
 }
 
@@ -676,9 +743,18 @@ struct FieldLayout {
 
 constexpr int kDirL = 32;
 constexpr int kDirTileRows = 32;
-constexpr int kDirStrips = kDirThreads / kDirTileRows;  // 8 strips of kDirL columns
+constexpr int kDirStrips = kDirThreads / kDirTileRows;  // strips of kDirL columns
 
 int field_gemm_splits(int64_t n, int h, int w);  // field_gemm.cu
+
+constexpr int kDirSmem = kBeamBatch * (int)(sizeof(BeamFast) + kDirL / 2 * sizeof(Ratio2));
+
+// Opted in once (before any capture that replays it).
+static cudaError_t dir_attr() {
+  static const cudaError_t done =
+      cudaFuncSetAttribute(k_field_direct<kDirL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDirSmem);
+  return done;
+}
 
 // Resident k_field_direct blocks per SM (register-limited), from the
 // occupancy calculator once per process.
@@ -686,7 +762,8 @@ static int dir_blocks_per_sm() {
   static int cached = 0;
   if (!cached) {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_field_direct<kDirL>, kDirThreads, 0) != cudaSuccess || b < 1)
+    if (dir_attr() != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_field_direct<kDirL>, kDirThreads, kDirSmem) != cudaSuccess || b < 1)
       b = 2;
     cached = b;
   }
@@ -862,7 +939,8 @@ extern "C" int tg_field_eval(int32_t method, int64_t n_beams, const tg_pixel_map
     int tiles = ((pm->h + kDirTileRows - 1) / kDirTileRows) *
                 ((pm->w + kDirStrips * kDirL - 1) / (kDirStrips * kDirL));
     int chunks = (int)((n_beams + A.chunk - 1) / A.chunk);
-    k_field_direct<kDirL><<<dim3(tiles, chunks), kDirThreads, 0, s>>>(A);
+    if (dir_attr() != cudaSuccess) return TG_ERR_CUDA;
+    k_field_direct<kDirL><<<dim3(tiles, chunks), kDirThreads, kDirSmem, s>>>(A);
     k_field_reduce<<<(int)((npx + 255) / 256), 256, 0, s>>>(part, chunks, npx, o);
   } else if (method == TG_FIELD_DIRECT_F64) {
     DirF64Args A;
@@ -974,7 +1052,8 @@ extern "C" int tg_field_direct_noalloc(const tg_model* model, const tg_beams* be
   const int tiles = ((pm->h + kDirTileRows - 1) / kDirTileRows) *
                     ((pm->w + kDirStrips * kDirL - 1) / (kDirStrips * kDirL));
   const int used = (int)((n + A.chunk - 1) / A.chunk);
-  k_field_direct<kDirL><<<dim3(tiles, used), kDirThreads, 0, s>>>(A);
+  if (dir_attr() != cudaSuccess) return TG_ERR_CUDA;
+  k_field_direct<kDirL><<<dim3(tiles, used), kDirThreads, kDirSmem, s>>>(A);
   k_field_reduce<<<(int)((npx + 255) / 256), 256, 0, s>>>(A.out, used, npx, o);
   return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
 }
