@@ -18,6 +18,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/temgym_gb300.h"
 #include "aberration.cuh"
 
@@ -212,7 +214,11 @@ __device__ __forceinline__ void hist_add_warp(CountT* hist, int bin, bool valid)
 __device__ __forceinline__ double f32_to_f64(float v) {
   const uint32_t b = __float_as_uint(v);
   const uint32_t e = (b >> 23) & 0xffu;
-  if (e == 0u || e == 0xffu) return (double)v;
+  if (e == 0u || e == 0xffu) {
+    double r;  // volatile: a plain cast is run for every thread, ahead of the branch
+    asm volatile("cvt.f64.f32 %0, %1;" : "=d"(r) : "f"(v));
+    return r;
+  }
   const uint64_t d = ((uint64_t)(b >> 31) << 63) | ((uint64_t)(e + (1023u - 127u)) << 52) |
                      ((uint64_t)(b & 0x7fffffu) << 29);
   return __longlong_as_double((long long)d);
@@ -618,6 +624,21 @@ __device__ __forceinline__ void op_reverse(const Op& op, const float4* pshift, R
     default:
       break;
   }
+}
+
+// Opts a kernel in to `bytes` (the same at every call) of dynamic shared memory,
+// once per device: before any capture that replays it.
+template <auto Kernel>
+static cudaError_t smem_opt_in(int bytes) {
+  static std::atomic<uint64_t> done{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = 1ull << (dev & 63);
+  if (done.load() & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done.fetch_or(bit);
+  return e;
 }
 
 }  // namespace tg

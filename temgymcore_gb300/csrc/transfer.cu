@@ -20,10 +20,18 @@ namespace tg {
 
 constexpr int kMaxTransfer = 120;  // matrices per call (24 KB of kernel parameters)
 
+// Zero pattern of a cumulative product: TR_FULL (none assumed), TR_AFFINE (last
+// row 0 0 0 0 c), TR_SPLIT (besides, x and y do not mix: rows x, dx use columns x,
+// dx, 1 and rows y, dy columns y, dy, 1; a column without a rotated element).  A
+// zero entry's product and sum are exact no-ops on a finite ray, so leaving them
+// out changes no result.
+enum TrClass : uint8_t { TR_FULL = 0, TR_AFFINE = 1, TR_SPLIT = 2 };
+
 struct TransferMats {
   int32_t m;
   int32_t pad;
   double c[kMaxTransfer][25];  // cumulative products, row-major
+  uint8_t cls[kMaxTransfer];   // TrClass of each
 };
 
 // ---------------------------------------------------------------- double-float
@@ -35,11 +43,6 @@ struct DF {
 __host__ __device__ inline bool df_range(double v) {
   const double a = v < 0 ? -v : v;
   return v == 0.0 || (a >= 1.8189894035458565e-12 && a <= 4.611686018427388e18);
-}
-
-__device__ __forceinline__ DF df_split(double v) {
-  const float h = __double2float_rn(v);
-  return DF{h, __double2float_rn(v - (double)h)};  // v - h is exact in float64
 }
 
 // a * b: the product of the heads with its exact rounding error, plus the
@@ -69,73 +72,216 @@ __device__ __forceinline__ DF df_norm(DF a) {
 }
 
 // hi + lo as a float64, faithfully rounded (within one float64 ulp: far below
-// the pair's own 2^-47), with a few integer operations.  For a renormalised
-// pair |lo| <= ulp32(hi) / 2, so in units of hi's float64 ulp lo is its
-// 24-bit significand shifted by sh = e_lo - e_hi + 29 <= 4, and the sum can
-// leave hi's binade only downwards and only when hi is a power of two: then
-// the grid below is twice as fine and lo counts double.  Zero, denormal and
-// non-finite parts take the general rounding.
-__device__ __forceinline__ double df_to_double(DF a) {
-  const uint32_t hb = __float_as_uint(a.h), lb = __float_as_uint(a.l);
-  const int eh = (int)((hb >> 23) & 0xffu), el = (int)((lb >> 23) & 0xffu);
-  if ((lb << 1) == 0u) return f32_to_f64(a.h);
-  if (eh == 0 || eh == 0xff || el == 0 || el == 0xff) return add_f64_f32(f32_to_f64(a.h), a.l);
-  const long long d = __double_as_longlong(f32_to_f64(a.h));
-  const uint32_t ml = (lb & 0x7fffffu) | 0x800000u;
-  const bool shrink = (hb >> 31) != (lb >> 31);  // lo reduces hi's magnitude
-  int sh = el - eh + 29;
-  if (shrink && (d & 0xfffffffffffffLL) == 0) ++sh;  // below a power of two: half-ulp grid
-  const long long n = sh >= 0 ? (long long)ml << sh : (sh > -25 ? (long long)(ml >> -sh) : 0LL);
-  return __longlong_as_double(d + (shrink ? -n : n));
+// the pair's own 2^-47), without float64 operations.  For a renormalised pair
+// |lo| <= ulp32(hi) / 2, so in units of hi's float64 ulp, 2^(e - 52), lo is a
+// number below 2^28: lo times the power of two, cut to an integer, is added to
+// hi's float64 bits.  A lo that reduces a power of two leaves hi's binade, where
+// the grid is twice as fine and lo counts double.  |hi| < 2^-75 (no such power of
+// two in float32; zero) and non-finite parts take the general rounding.
+__device__ __forceinline__ double df_to_double(float h, float l) {
+  const uint32_t hb = __float_as_uint(h), lb = __float_as_uint(l);
+  if ((hb & 0x7fffffffu) - (52u << 23) >= (203u << 23)) {
+    if ((hb << 1) == 0u) return __longlong_as_double((long long)((uint64_t)(hb + lb) << 32));  // lo is 0 too
+    return add_f64_f32(f32_to_f64(h), l);
+  }
+  uint32_t scale = 0x99000000u - (hb & 0xff800000u);  // 2^(52 - e) with hi's sign
+  if ((hb & 0x7fffffu) == 0u && (int32_t)(hb ^ lb) < 0) scale += 1u << 23;
+  const int n = __float2int_rz(__fmul_rn(l, __uint_as_float(scale)));
+  // hi's float64 bits: exponent rebiased (+ 896 << 20), significand widened
+  const uint32_t dhi = (uint32_t)((((int32_t)hb >> 3) & (int32_t)0x8fffffff) + 0x38000000), dlo = hb << 29;
+  return __longlong_as_double((long long)(((uint64_t)dhi << 32) | dlo) + (long long)n);
 }
 
-constexpr int kTrRays = 64;  // rays staged per block iteration
+// ------------------------------------------------- two double-floats at a time
+// Packed pairs of float32 (the component of x and the component of y): one
+// instruction issues both, and each half rounds as the scalar operation does.
+struct F2 {
+  unsigned long long u;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+  return F2{((unsigned long long)__float_as_uint(b) << 32) | __float_as_uint(a)};
+}
+__device__ __forceinline__ float f2_lo(F2 a) { return __uint_as_float((uint32_t)a.u); }
+__device__ __forceinline__ float f2_hi(F2 a) { return __uint_as_float((uint32_t)(a.u >> 32)); }
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.u) : "l"(a.u), "l"(b.u));
+  return d;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.u) : "l"(a.u), "l"(b.u), "l"(c.u));
+  return d;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.u) : "l"(a.u), "l"(b.u));
+  return d;
+}
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {
+  F2 d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d.u) : "l"(a.u), "l"(b.u));
+  return d;
+}
 
-// out[n][p][i] = sum_j C[p][i][j] ray[n][j] in double-float.  A block splits
-// the matrices into float32 pairs once, then per group of kTrRays rays stages
-// their split components in shared memory (the split is shared by all
-// planes) and runs one (ray, plane) pair per thread: a warp writes 32
-// consecutive 40-byte records.
-__global__ void __launch_bounds__(256)
-k_transfer_rays_df(const __grid_constant__ TransferMats T, int64_t n, const double* __restrict__ rays,
-                   double* __restrict__ out) {
-  extern __shared__ DF tsm[];  // [m * 25] matrix pairs, then [kTrRays * 5] ray pairs
-  __shared__ int s_ok[kTrRays];
-  const int m = T.m;
-  DF* mc = tsm;
-  DF* rv = tsm + m * 25;
-  for (int i = threadIdx.x; i < m * 25; i += blockDim.x) mc[i] = df_split((&T.c[0][0])[i]);
-  for (int64_t g = (int64_t)blockIdx.x * kTrRays; g < n; g += (int64_t)gridDim.x * kTrRays) {
-    const int nr = (int)((n - g) < kTrRays ? (n - g) : kTrRays);
-    __syncthreads();  // the previous group's pairs are done with rv / s_ok
-    for (int i = threadIdx.x; i < nr * 5; i += blockDim.x) rv[i] = df_split(rays[g * 5 + i]);
-    for (int i = threadIdx.x; i < nr; i += blockDim.x) {
-      const double* v = rays + (g + i) * 5;
-      s_ok[i] = df_range(v[0]) && df_range(v[1]) && df_range(v[2]) && df_range(v[3]) && df_range(v[4]);
+// A pair of ray components, with the negated parts that the products below use.
+struct Ray2 {
+  F2 h, nh, nl;
+};
+__device__ __forceinline__ Ray2 ray2(DF a, DF b) {
+  return Ray2{f2(a.h, b.h), f2(-a.h, -b.h), f2(-a.l, -b.l)};
+}
+// A pair of double-floats as (hi, -lo): the error of a product then needs no
+// negation, h v - p = -(p + h (-v)).
+struct DF2 {
+  F2 h, nl;
+};
+__device__ __forceinline__ DF2 df2_mul(const ulonglong2& c, const Ray2& v) {  // c = (hi, hi), (lo, lo)
+  const F2 ch{c.x}, cl{c.y};
+  const F2 p = f2_mul(ch, v.h);
+  return DF2{p, f2_fma(cl, v.nh, f2_fma(ch, v.nl, f2_fma(ch, v.nh, p)))};
+}
+__device__ __forceinline__ DF2 df2_add(DF2 a, DF2 b) {  // df_add
+  const F2 s = f2_add(a.h, b.h), bb = f2_sub(s, a.h);
+  const F2 err = f2_add(f2_sub(a.h, f2_sub(s, bb)), f2_sub(b.h, bb));
+  return DF2{s, f2_sub(f2_add(a.nl, b.nl), err)};
+}
+
+// The split of a float64 inside the double-float range, with integer operations:
+// the head is the value rounded to 24 bits (ties away from zero), the tail the
+// signed rest in units of 2^(e - 52), rounded to 24 bits.  False for a value
+// outside the range (2^62 itself too), whose split means nothing.
+__device__ __forceinline__ bool df_component(double v, DF& out) {
+  const uint64_t b = (uint64_t)__double_as_longlong(v);
+  const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b, e = (hi >> 20) & 0x7ffu, sign = hi & 0x80000000u;
+  const uint32_t top = ((hi & 0x7fffffffu) << 3 | lo >> 29) - (896u << 23);  // exponent and 23 bits
+  const int rest = (int)(lo << 3) >> 3;                                       // the low 29 bits, signed
+  const bool zero = ((hi << 1) | lo) == 0u;
+  out.h = zero ? 0.0f : __uint_as_float(sign | (top + ((lo >> 28) & 1u)));
+  out.l = zero ? 0.0f : __fmul_rn(__int2float_rn(rest), __uint_as_float(sign | ((e - 948u) << 23)));
+  return zero || e - (1023u - 39u) < 101u;
+}
+
+constexpr int kTrThreads = 256;
+constexpr int kTrMinBlocks = 4;
+constexpr int kTrWaves = 4;       // blocks per SM and wave aimed at
+constexpr int kTrPlanes = 4;      // planes between two writes
+constexpr int kTrStride = 22;     // doubles per ray in a warp's buffer: 4 records of 5, 16-byte aligned
+constexpr int kTrWarpDoubles = 32 * kTrStride;
+constexpr int kTrVec = 5 * kTrPlanes / 2;    // 16-byte vectors of a ray's records
+constexpr int kTrWriteRays = 32 / kTrVec;    // whole rays in a warp's write
+static_assert(kTrPlanes % 2 == 0 && kTrStride % 2 == 0 && kTrStride >= 5 * kTrPlanes && kTrWriteRays >= 1, "");
+constexpr int kTrTab = 13;        // 16-byte entries of a plane's split matrix
+
+// out[n][p][i] = sum_j C[p][i][j] ray[n][j] in double-float.  A thread keeps one
+// ray's split components in registers and walks planes [p0, p1) of its block
+// row, so that a warp reads each matrix entry once (a broadcast) and skips a
+// plane's zero entries together.  The rows of x and y (and of dx and dy) are a
+// packed pair: row x takes columns x, y, dx, dy, 1 and row y columns y, x, dy,
+// dx, 1.  Four planes' records of the warp's rays are collected in shared memory
+// and leave as 16-byte vectors, 160 contiguous bytes a ray.  Bound by the
+// instructions issued (8 a term and pair, 20 to round a result).  Measured at
+// 1 M rays x 16 planes (6 planes split, 10 affine): 208 us; 399 with one
+// (ray, plane) pair per thread, 25 terms each, and a float64 conversion run for
+// every result ahead of its branch (52 % of the float64 pipe).
+__global__ void __launch_bounds__(kTrThreads, kTrMinBlocks)
+k_transfer_rays_df(const __grid_constant__ TransferMats T, int64_t n, int planes_per_block,
+                   const double* __restrict__ rays, double* __restrict__ out, int vec) {
+  extern __shared__ __align__(16) double trm[];  // [warps][32][kTrStride] records, then the planes' split matrices
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int p0 = blockIdx.y * planes_per_block, p1 = min(T.m, p0 + planes_per_block);
+  double* rec = trm + warp * kTrWarpDoubles;
+  ulonglong2* mc = reinterpret_cast<ulonglong2*>(trm + kTrThreads / 32 * kTrWarpDoubles);
+  // entries 0..4: rows x and y, 5..9: rows dx and dy, 10..12: the last row's five
+  for (int i = threadIdx.x; i < (p1 - p0) * kTrTab; i += kTrThreads) {
+    const int p = i / kTrTab, e = i - p * kTrTab;
+    const double* c = T.c[p0 + p];
+    double a, b;
+    if (e < 10) {
+      const int row = e < 5 ? 0 : 2, j = e < 5 ? e : e - 5;
+      a = c[row * 5 + j];
+      b = c[row * 5 + 5 + (j == 4 ? 4 : j ^ 1)];
+    } else {
+      const int j = (e - 10) * 2;
+      a = c[20 + j];
+      b = j < 4 ? c[21 + j] : 0.0;
     }
-    __syncthreads();
-    const int pairs = nr * m;
-    for (int q = threadIdx.x; q < pairs; q += blockDim.x) {
-      const int r = q / m, p = q - r * m;
-      double* o = out + ((g + r) * m + p) * 5;
-      if (s_ok[r]) {
-        const DF* c = mc + p * 25;
-        const DF* v = rv + r * 5;
+    DF da, db;  // in range: the host's rule
+    df_component(a, da);
+    df_component(b, db);
+    mc[i] = make_ulonglong2(f2(da.h, db.h).u, f2(da.l, db.l).u);
+  }
+  __syncthreads();
+  const int sub = lane / kTrVec, off = lane - sub * kTrVec;  // a write takes the records of kTrWriteRays rays
+  const int64_t stride = (int64_t)gridDim.x * kTrThreads;
+  for (int64_t r0 = (int64_t)blockIdx.x * kTrThreads + warp * 32; r0 < n; r0 += stride) {  // the warp's 32 rays
+    const int64_t r = r0 + lane;
+    const double* src = rays + 5 * (r < n ? r : n - 1);
+    DF v[5];
+    bool ok = true;
 #pragma unroll
-        for (int i = 0; i < 5; ++i) {
-          DF acc = df_mul(c[5 * i], v[0]);
+    for (int j = 0; j < 5; ++j) ok &= df_component(__ldg(src + j), v[j]);
+    const Ray2 xy = ray2(v[0], v[1]), yx = ray2(v[1], v[0]), sxy = ray2(v[2], v[3]), syx = ray2(v[3], v[2]),
+               one = ray2(v[4], v[4]);
+    const int live = (int)(n - r0 < 32 ? n - r0 : 32);
+    for (int pc = p0; pc < p1; pc += kTrPlanes) {
+      const int np = min(kTrPlanes, p1 - pc);
+      for (int q = 0; q < np; ++q) {
+        const ulonglong2* c = mc + (pc - p0 + q) * kTrTab;
+        double* o = rec + lane * kTrStride + 5 * q;
+        const int cls = T.cls[pc + q];  // the same for the whole block
 #pragma unroll
-          for (int j = 1; j < 5; ++j) acc = df_add(acc, df_mul(c[5 * i + j], v[j]));
-          o[i] = df_to_double(df_norm(acc));
+        for (int i = 0; i < 2; ++i) {
+          DF2 a = df2_mul(c[5 * i], xy);
+          if (cls == TR_SPLIT) {
+            a = df2_add(a, df2_mul(c[5 * i + 2], sxy));
+          } else {
+            a = df2_add(a, df2_mul(c[5 * i + 1], yx));
+            a = df2_add(a, df2_mul(c[5 * i + 2], sxy));
+            a = df2_add(a, df2_mul(c[5 * i + 3], syx));
+          }
+          a = df2_add(a, df2_mul(c[5 * i + 4], one));
+          const F2 h = f2_sub(a.h, a.nl);  // df_norm
+          const F2 nl = f2_add(a.nl, f2_sub(h, a.h));
+          o[2 * i] = df_to_double(f2_lo(h), -f2_lo(nl));
+          o[2 * i + 1] = df_to_double(f2_hi(h), -f2_hi(nl));
         }
-      } else {  // outside the double-float range: float64
-        const double* v = rays + (g + r) * 5;
-        const double* c = T.c[p];
+        const float* cf = reinterpret_cast<const float*>(c + 10);  // h, h, l, l of two entries
+        DF acc = df_mul(DF{cf[8], cf[10]}, v[4]);
+        if (cls == TR_FULL) {
+          DF sum = df_mul(DF{cf[0], cf[2]}, v[0]);
 #pragma unroll
-        for (int i = 0; i < 5; ++i)
-          o[i] = c[5 * i + 0] * v[0] + c[5 * i + 1] * v[1] + c[5 * i + 2] * v[2] +
-                 c[5 * i + 3] * v[3] + c[5 * i + 4] * v[4];
+          for (int j = 1; j < 4; ++j)
+            sum = df_add(sum, df_mul(DF{cf[(j >> 1) * 4 + (j & 1)], cf[(j >> 1) * 4 + 2 + (j & 1)]}, v[j]));
+          acc = df_add(sum, acc);
+        }
+        acc = df_norm(acc);
+        o[4] = df_to_double(acc.h, acc.l);
+        if (!ok) {  // outside the double-float range: float64
+          const double* c64 = T.c[pc + q];
+#pragma unroll 1
+          for (int i = 0; i < 5; ++i)
+            o[i] = c64[5 * i + 0] * src[0] + c64[5 * i + 1] * src[1] + c64[5 * i + 2] * src[2] +
+                   c64[5 * i + 3] * src[3] + c64[5 * i + 4] * src[4];
+        }
       }
+      __syncwarp();
+      const int64_t pitch = (int64_t)T.m * 5;
+      double* dst = out + r0 * pitch + pc * 5;
+      if (vec && np == kTrPlanes) {  // m and pc even, out 16-byte aligned
+        const double* from = rec + sub * kTrStride + 2 * off;
+        double* to = dst + sub * pitch + 2 * off;
+        for (int ray = sub; ray < live && sub < kTrWriteRays;
+             ray += kTrWriteRays, from += kTrWriteRays * kTrStride, to += kTrWriteRays * pitch)
+          *reinterpret_cast<double2*>(to) = *reinterpret_cast<const double2*>(from);
+      } else {
+        const int per = 5 * np;  // doubles of a ray
+        for (int i = lane; i < live * per; i += 32) {
+          const int ray = i / per, k = i - ray * per;
+          dst[(int64_t)ray * pitch + k] = rec[ray * kTrStride + k];
+        }
+      }
+      __syncwarp();
     }
   }
 }
@@ -242,11 +388,28 @@ extern "C" int tg_transfer_rays(int64_t n, const double* rays, int32_t m, const 
   bool df = true;
   for (int i = 0; i < m * 25 && df; ++i) df = df_range((&T.c[0][0])[i]);
   if (df) {
-    const size_t smem = (size_t)(m * 25 + kTrRays * 5) * sizeof(DF);  // <= 26.6 KB
-    int64_t blocks = (n + kTrRays - 1) / kTrRays;
-    const int64_t cap = (int64_t)sm_count_transfer() * 8;
-    if (blocks > cap) blocks = cap;
-    k_transfer_rays_df<<<(int)blocks, 256, smem, s>>>(T, n, rays, out);
+    for (int p = 0; p < m; ++p) {
+      const double* c = T.c[p];
+      auto zero = [&](int i, int j) { return c[5 * i + j] == 0.0; };
+      bool affine = true, split = true;
+      for (int j = 0; j < 4; ++j) affine = affine && zero(4, j);
+      for (int i = 0; i < 4; ++i) split = split && zero(i, 1 - (i & 1)) && zero(i, 3 - (i & 1));
+      T.cls[p] = affine ? (split ? TR_SPLIT : TR_AFFINE) : TR_FULL;
+    }
+    // all planes a thread where the rays fill the GPU, else fewer (a multiple
+    // of kTrPlanes) over more blocks
+    const int64_t rblocks = (n + kTrThreads - 1) / kTrThreads, want = (int64_t)sm_count_transfer() * 4 * kTrWaves;
+    int64_t rows = (want + rblocks - 1) / rblocks;
+    const int groups = (m + kTrPlanes - 1) / kTrPlanes;
+    if (rows > groups) rows = groups;
+    const int per = (int)((groups + rows - 1) / rows) * kTrPlanes;
+    const size_t smem = sizeof(double) * (kTrThreads / 32) * kTrWarpDoubles +
+                        sizeof(ulonglong2) * kTrTab * (size_t)(per < m ? per : m);  // at most 70 KB
+    const int smem_max = (int)(sizeof(double) * (kTrThreads / 32) * kTrWarpDoubles + sizeof(ulonglong2) * kTrTab * kMaxTransfer);
+    if (smem_opt_in<k_transfer_rays_df>(smem_max) != cudaSuccess) return TG_ERR_CUDA;
+    const int vec = (m & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    const dim3 grid((unsigned)(rblocks < want ? rblocks : want), (unsigned)((m + per - 1) / per));
+    k_transfer_rays_df<<<grid, kTrThreads, smem, s>>>(T, n, per, rays, out, vec);
     return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
   }
   const int64_t total = n * (int64_t)m;
