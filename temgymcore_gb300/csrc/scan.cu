@@ -420,10 +420,7 @@ static bool scan_use_image(int64_t n, size_t smem) {
 
 template <int T, int kPerSm>
 static int scan_image_launch(const Program& P, const ScanArgs& A, const BinCoef& B, size_t smem, cudaStream_t s) {
-  // opted in once per instantiation (before any capture that replays it)
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      k_scan_image<T, kPerSm>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem_max());
-  if (attr != cudaSuccess) return TG_ERR_CUDA;
+  if (smem_opt_in<k_scan_image<T, kPerSm>>((int)scan_smem_max()) != cudaSuccess) return TG_ERR_CUDA;
   const int res = sm_count_scan() * kPerSm;
   k_scan_image<T, kPerSm><<<res < A.n_probes ? res : A.n_probes, T, smem, s>>>(P, A, B);
   return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
@@ -486,9 +483,7 @@ extern "C" int tg_scan_hist(const tg_model* model, const tg_rays* bundle, const 
     return scan_image_launch<1024, 1>(P, A, B, img_smem, s);
   }
   A.win_bins = (kHistSmem - kZeroBytes - (A.n <= kMaxSmemRays ? (int)(A.n + 3) / 4 * 16 : 0)) / 4 * 2;
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(k_scan_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, kHistSmem);
-  if (attr != cudaSuccess) return TG_ERR_CUDA;
+  if (smem_opt_in<k_scan_hist>(kHistSmem) != cudaSuccess) return TG_ERR_CUDA;
   static int per_sm = 0;  // residency, queried once
   if (!per_sm) {
     int q = 0;
