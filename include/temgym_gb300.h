@@ -639,6 +639,14 @@ int tg_field_prep_input(const tg_beams *beams, const tg_pixel_map *pm, void *wor
 int tg_field_eval(int32_t method, int64_t n_beams, const tg_pixel_map *pm, float *out,
                   void *workspace, size_t ws_bytes, void *stream);
 
+/* tg_field_eval with the method picked on the device by the preparation's flags
+ * (tg_field_prep's device int32): separable when bit 0 is clear, else direct.
+ * Both are launched and one works; the host does not wait.  ws_bytes: the larger
+ * of the two methods' workspaces.  TG_ERR_TOO_LARGE: more pixels a side or beams
+ * than the separable method takes. */
+int tg_field_eval_auto(int64_t n_beams, const tg_pixel_map *pm, const int32_t *flags, float *out,
+                       void *workspace, size_t ws_bytes, void *stream);
+
 /* tg_field_prep + tg_field_eval(TG_FIELD_DIRECT / TG_FIELD_SEPARABLE) in one
  * call; workspace as for tg_field_eval with that method. */
 int tg_field_direct(const tg_model *model, const tg_beams *beams, const tg_pixel_map *pm,

@@ -323,6 +323,15 @@ k_field_prep(const __grid_constant__ DModel M, const __grid_constant__ PrepArgs 
   if (k_rc.re != 0.0 || k_rc.im != 0.0) atomicOr(A.flags, 1);
 }
 
+// The preparation's status word decides on the device which of the two methods'
+// kernels work (tg_field_eval_auto launches both): a kernel of the other method
+// returns at once.  No flag: no decision.
+struct FieldGate {
+  const int32_t* flags;  // != 0: some beam is not separable
+  int32_t direct;        // this kernel is of the direct method
+  __device__ __forceinline__ bool closed() const { return flags && (__ldg(flags) != 0) != (direct != 0); }
+};
+
 // ---------------------------------------------------------------- direct
 constexpr int kDirThreads = 256;
 constexpr int kBeamBatch = 128;
@@ -335,6 +344,7 @@ struct DirArgs {
   int32_t tile_rows;   // rows per tile
   int32_t strips_x;    // strips per tile row
   float2* out;         // [gridDim.y][h][w] partials (or the image if gridDim.y == 1)
+  FieldGate gate;
 };
 
 // Per (beam, strip) the log-amplitude decides how the strip is summed: skip
@@ -388,6 +398,7 @@ __global__ void __launch_bounds__(kDirThreads, 2)
 k_field_direct(const __grid_constant__ DirArgs A) {
   static_assert(L % kDirRestart == 0 && kDirRestart % 2 == 0, "whole pixel pairs between restarts");
   constexpr int H = L / 2;
+  if (A.gate.closed()) return;
   extern __shared__ __align__(16) unsigned char dir_smem[];  // the batch's records, then its ratio tables
   BeamFast* sb = reinterpret_cast<BeamFast*>(dir_smem);
   Ratio2 (*tab)[H] = reinterpret_cast<Ratio2 (*)[H]>(dir_smem + kBeamBatch * sizeof(BeamFast));
@@ -557,10 +568,8 @@ k_field_direct_f64(const __grid_constant__ DirF64Args A) {
   if (p < npx) A.out[(size_t)blockIdx.y * npx + p] = make_float2((float)sr, (float)si);
 }
 
-__global__ void k_field_reduce(const float2* __restrict__ part, int nchunk, int64_t npx,
-                               float2* __restrict__ out) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= npx) return;
+__device__ __forceinline__ void reduce_pixel(const float2* __restrict__ part, int nchunk, int64_t npx,
+                                             float2* __restrict__ out, int64_t i) {
   float sr = 0.f, si = 0.f;
   for (int c = 0; c < nchunk; ++c) {
     float2 v = part[(size_t)c * npx + i];
@@ -568,6 +577,22 @@ __global__ void k_field_reduce(const float2* __restrict__ part, int nchunk, int6
     si += v.y;
   }
   out[i] = make_float2(sr, si);
+}
+
+__global__ void k_field_reduce(const float2* __restrict__ part, int nchunk, int64_t npx,
+                               float2* __restrict__ out) {
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= npx) return;
+  reduce_pixel(part, nchunk, npx, out, i);
+}
+
+// Either method's partials, by the preparation's status word.
+__global__ void k_field_reduce_auto(const int32_t* flags, const float2* __restrict__ sep, int nsep,
+                                    const float2* __restrict__ dir, int ndir, int64_t npx, float2* __restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= npx) return;
+  const bool direct = __ldg(flags) != 0;
+  reduce_pixel(direct ? dir : sep, direct ? ndir : nsep, npx, out, i);
 }
 
 // ---------------------------------------------------------------- operands
@@ -583,6 +608,7 @@ struct OperandArgs {
   int32_t h, w;
   __nv_bfloat16_raw* v_planes;  // 4 * lines_v * kpad
   __nv_bfloat16_raw* u_planes;  // 4 * lines_u * kpad
+  FieldGate gate;
 };
 
 }  // namespace tg
@@ -599,6 +625,7 @@ namespace tg {
 constexpr int kOpLines = 32;  // measured (16,384 beams, 512^2, whole evaluation): 8 lines 0.108 ms, 16 0.0998, 32 0.0982, 64 0.0977
 
 __global__ void __launch_bounds__(256) k_field_operands(const __grid_constant__ OperandArgs A) {
+  if (A.gate.closed()) return;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= A.kpad) return;
   const int vblocks = A.lines_v / kOpLines;
@@ -749,12 +776,7 @@ int field_gemm_splits(int64_t n, int h, int w);  // field_gemm.cu
 
 constexpr int kDirSmem = kBeamBatch * (int)(sizeof(BeamFast) + kDirL / 2 * sizeof(Ratio2));
 
-// Opted in once (before any capture that replays it).
-static cudaError_t dir_attr() {
-  static const cudaError_t done =
-      cudaFuncSetAttribute(k_field_direct<kDirL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDirSmem);
-  return done;
-}
+static cudaError_t dir_attr() { return smem_opt_in<k_field_direct<kDirL>>(kDirSmem); }
 
 // Resident k_field_direct blocks per SM (register-limited), from the
 // occupancy calculator once per process.
@@ -821,7 +843,7 @@ static FieldLayout field_layout(int64_t n, int h, int w, int method) {
 
 int launch_field_gemm(const __nv_bfloat16_raw* vplanes, const __nv_bfloat16_raw* uplanes,
                       int lines_v, int lines_u, int64_t kpad, int splits, int h, int w,
-                      float2* part, cudaStream_t s);  // field_gemm.cu
+                      float2* part, cudaStream_t s, const int32_t* flags = nullptr);  // field_gemm.cu
 
 static bool field_method_ok(int method) {
   return method == TG_FIELD_DIRECT || method == TG_FIELD_SEPARABLE || method == TG_FIELD_DIRECT_F64;
@@ -910,6 +932,52 @@ extern "C" int tg_field_prep_input(const tg_beams* beams, const tg_pixel_map* pm
   return field_prep_launch(dm, beams, pm, workspace, ws_bytes, flags, stream, 1);
 }
 
+// The direct and the separable sum's partials (L: that method's layout; flags:
+// FieldGate's, or null).  chunks: the partial images written.
+static int launch_direct_part(const FieldLayout& L, int64_t n_beams, const tg_pixel_map* pm, char* ws,
+                              const int32_t* flags, int* chunks, cudaStream_t s) {
+  DirArgs A;
+  A.beams = reinterpret_cast<const BeamFast*>(ws + L.fast);
+  A.n = n_beams;
+  A.chunk = (n_beams + L.chunks - 1) / L.chunks;
+  A.h = pm->h;
+  A.w = pm->w;
+  A.tile_rows = kDirTileRows;
+  A.strips_x = kDirStrips;
+  A.out = reinterpret_cast<float2*>(ws + L.part);
+  A.gate = FieldGate{flags, 1};
+  int tiles = ((pm->h + kDirTileRows - 1) / kDirTileRows) *
+              ((pm->w + kDirStrips * kDirL - 1) / (kDirStrips * kDirL));
+  *chunks = (int)((n_beams + A.chunk - 1) / A.chunk);
+  if (dir_attr() != cudaSuccess) return TG_ERR_CUDA;
+  k_field_direct<kDirL><<<dim3(tiles, *chunks), kDirThreads, kDirSmem, s>>>(A);
+  return TG_OK;
+}
+
+static bool separable_too_large(const FieldLayout& L) {
+  return L.lines_v % kOpLines || L.lines_u % kOpLines || L.kpad > INT32_MAX;
+}
+
+static int launch_separable_part(const FieldLayout& L, int64_t n_beams, const tg_pixel_map* pm, char* ws,
+                                 const int32_t* flags, cudaStream_t s) {
+  OperandArgs A;
+  A.beams = reinterpret_cast<const BeamFast*>(ws + L.fast);
+  A.n = n_beams;
+  A.kpad = L.kpad;
+  A.lines_v = L.lines_v;
+  A.lines_u = L.lines_u;
+  A.h = pm->h;
+  A.w = pm->w;
+  A.v_planes = reinterpret_cast<__nv_bfloat16_raw*>(ws + L.vplanes);
+  A.u_planes = reinterpret_cast<__nv_bfloat16_raw*>(ws + L.uplanes);
+  A.gate = FieldGate{flags, 0};
+  if (separable_too_large(L)) return TG_ERR_TOO_LARGE;
+  k_field_operands<<<dim3((unsigned)((L.kpad + 255) / 256), (unsigned)((L.lines_v + L.lines_u) / kOpLines)), 256,
+                     0, s>>>(A);
+  return launch_field_gemm(A.v_planes, A.u_planes, L.lines_v, L.lines_u, L.kpad, L.chunks, pm->h, pm->w,
+                           reinterpret_cast<float2*>(ws + L.part), s, flags);
+}
+
 extern "C" int tg_field_eval(int32_t method, int64_t n_beams, const tg_pixel_map* pm,
                              float* out, void* workspace, size_t ws_bytes, void* stream) {
   if (!pm || pm->h <= 0 || pm->w <= 0 || n_beams < 0 || !out) return TG_ERR_INVALID;
@@ -927,20 +995,9 @@ extern "C" int tg_field_eval(int32_t method, int64_t n_beams, const tg_pixel_map
   }
   float2* part = reinterpret_cast<float2*>(ws + L.part);
   if (method == TG_FIELD_DIRECT) {
-    DirArgs A;
-    A.beams = reinterpret_cast<const BeamFast*>(ws + L.fast);
-    A.n = n_beams;
-    A.chunk = (n_beams + L.chunks - 1) / L.chunks;
-    A.h = pm->h;
-    A.w = pm->w;
-    A.tile_rows = kDirTileRows;
-    A.strips_x = kDirStrips;
-    A.out = part;
-    int tiles = ((pm->h + kDirTileRows - 1) / kDirTileRows) *
-                ((pm->w + kDirStrips * kDirL - 1) / (kDirStrips * kDirL));
-    int chunks = (int)((n_beams + A.chunk - 1) / A.chunk);
-    if (dir_attr() != cudaSuccess) return TG_ERR_CUDA;
-    k_field_direct<kDirL><<<dim3(tiles, chunks), kDirThreads, kDirSmem, s>>>(A);
+    int chunks = 0;
+    int st = launch_direct_part(L, n_beams, pm, ws, nullptr, &chunks, s);
+    if (st != TG_OK) return st;
     k_field_reduce<<<(int)((npx + 255) / 256), 256, 0, s>>>(part, chunks, npx, o);
   } else if (method == TG_FIELD_DIRECT_F64) {
     DirF64Args A;
@@ -954,24 +1011,33 @@ extern "C" int tg_field_eval(int32_t method, int64_t n_beams, const tg_pixel_map
     k_field_direct_f64<<<dim3((unsigned)((npx + 255) / 256), chunks), 256, 0, s>>>(A);
     k_field_reduce<<<(int)((npx + 255) / 256), 256, 0, s>>>(part, chunks, npx, o);
   } else {
-    OperandArgs A;
-    A.beams = reinterpret_cast<const BeamFast*>(ws + L.fast);
-    A.n = n_beams;
-    A.kpad = L.kpad;
-    A.lines_v = L.lines_v;
-    A.lines_u = L.lines_u;
-    A.h = pm->h;
-    A.w = pm->w;
-    A.v_planes = reinterpret_cast<__nv_bfloat16_raw*>(ws + L.vplanes);
-    A.u_planes = reinterpret_cast<__nv_bfloat16_raw*>(ws + L.uplanes);
-    if (L.lines_v % kOpLines || L.lines_u % kOpLines || L.kpad > INT32_MAX) return TG_ERR_TOO_LARGE;
-    k_field_operands<<<dim3((unsigned)((L.kpad + 255) / 256), (unsigned)((L.lines_v + L.lines_u) / kOpLines)), 256,
-                       0, s>>>(A);
-    int st = launch_field_gemm(A.v_planes, A.u_planes, L.lines_v, L.lines_u, L.kpad, L.chunks,
-                               pm->h, pm->w, part, s);
+    int st = launch_separable_part(L, n_beams, pm, ws, nullptr, s);
     if (st != TG_OK) return st;
     k_field_reduce<<<(int)((npx + 255) / 256), 256, 0, s>>>(part, L.chunks, npx, o);
   }
+  return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
+}
+
+extern "C" int tg_field_eval_auto(int64_t n_beams, const tg_pixel_map* pm, const int32_t* flags, float* out,
+                                  void* workspace, size_t ws_bytes, void* stream) {
+  if (!pm || pm->h <= 0 || pm->w <= 0 || n_beams < 0 || !out || !flags) return TG_ERR_INVALID;
+  const FieldLayout D = field_layout(n_beams, pm->h, pm->w, TG_FIELD_DIRECT);
+  const FieldLayout S = field_layout(n_beams, pm->h, pm->w, TG_FIELD_SEPARABLE);
+  if (!workspace || ws_bytes < D.total || ws_bytes < S.total) return TG_ERR_WORKSPACE;
+  if (((uintptr_t)workspace & 255) != 0) return TG_ERR_ALIGN;
+  if (separable_too_large(S) || (S.lines_v + S.lines_u) / kOpLines > 65535) return TG_ERR_TOO_LARGE;  // grid.y
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  char* ws = reinterpret_cast<char*>(workspace);
+  const int64_t npx = (int64_t)pm->h * pm->w;
+  if (n_beams == 0)
+    return cudaMemsetAsync(out, 0, (size_t)npx * sizeof(float2), s) == cudaSuccess ? TG_OK : TG_ERR_CUDA;
+  int chunks = 0;
+  int st = launch_separable_part(S, n_beams, pm, ws, flags, s);
+  if (st == TG_OK) st = launch_direct_part(D, n_beams, pm, ws, flags, &chunks, s);
+  if (st != TG_OK) return st;
+  k_field_reduce_auto<<<(int)((npx + 255) / 256), 256, 0, s>>>(
+      flags, reinterpret_cast<const float2*>(ws + S.part), S.chunks, reinterpret_cast<const float2*>(ws + D.part),
+      chunks, npx, reinterpret_cast<float2*>(out));
   return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
 }
 
@@ -1040,21 +1106,12 @@ extern "C" int tg_field_direct_noalloc(const tg_model* model, const tg_beams* be
   const int64_t fit = (int64_t)((kNoAllocBytes - L.part) / per_chunk);
   if (chunks > fit) chunks = fit;
   char* ws = reinterpret_cast<char*>(scratch);
-  DirArgs A;
-  A.beams = reinterpret_cast<const BeamFast*>(ws + L.fast);
-  A.n = n;
-  A.chunk = (n + chunks - 1) / chunks;
-  A.h = pm->h;
-  A.w = pm->w;
-  A.tile_rows = kDirTileRows;
-  A.strips_x = kDirStrips;
-  A.out = reinterpret_cast<float2*>(ws + L.part);  // every in-range pixel is overwritten
-  const int tiles = ((pm->h + kDirTileRows - 1) / kDirTileRows) *
-                    ((pm->w + kDirStrips * kDirL - 1) / (kDirStrips * kDirL));
-  const int used = (int)((n + A.chunk - 1) / A.chunk);
-  if (dir_attr() != cudaSuccess) return TG_ERR_CUDA;
-  k_field_direct<kDirL><<<dim3(tiles, used), kDirThreads, kDirSmem, s>>>(A);
-  k_field_reduce<<<(int)((npx + 255) / 256), 256, 0, s>>>(A.out, used, npx, o);
+  FieldLayout C = L;  // every in-range pixel of a partial image is overwritten
+  C.chunks = (int)chunks;
+  int used = 0;
+  st = launch_direct_part(C, n, pm, ws, nullptr, &used, s);
+  if (st != TG_OK) return st;
+  k_field_reduce<<<(int)((npx + 255) / 256), 256, 0, s>>>(reinterpret_cast<const float2*>(ws + L.part), used, npx, o);
   return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
 }
 

@@ -1072,7 +1072,7 @@ extern "C" size_t tg_field_vjp_workspace_ex(int32_t method, int64_t n_beams, int
 namespace tg {
 int launch_field_gemm(const __nv_bfloat16_raw* vplanes, const __nv_bfloat16_raw* uplanes, int lines_v,
                       int lines_u, int64_t kpad, int splits, int h, int w, float2* part,
-                      cudaStream_t s);  // field_gemm.cu
+                      cudaStream_t s, const int32_t* flags = nullptr);  // field_gemm.cu
 }
 
 static int field_vjp_impl(const tg_model* model, const tg_beams* beams, const tg_pixel_map* pm,

@@ -93,10 +93,12 @@ struct GemmArgs {
   int32_t nkb;     // K blocks (of 32) per split
   int32_t h, w;
   float2* part;    // [splits][h][w]
+  const int32_t* flags;  // when given and != 0 (beams not separable): nothing to do
 };
 
 __global__ void __launch_bounds__(128, 1)
 k_field_gemm(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmArgs A) {
+  if (A.flags && __ldg(A.flags) != 0) return;  // the whole grid: before any barrier or TMEM
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kGStages * kStageBytes);
@@ -259,7 +261,7 @@ int field_gemm_splits(int64_t n, int h, int w) {
 
 int launch_field_gemm(const __nv_bfloat16_raw* vplanes, const __nv_bfloat16_raw* uplanes, int lines_v,
                       int lines_u, int64_t kpad, int splits, int h, int w, float2* part,
-                      cudaStream_t s) {
+                      cudaStream_t s, const int32_t* flags) {
   // the eight tensor maps of a plane buffer, encoded once per (buffers,
   // shape) and kept in a small round-robin cache (an evaluation cycles through
   // two buffers; a few plans may alternate)
@@ -300,6 +302,7 @@ int launch_field_gemm(const __nv_bfloat16_raw* vplanes, const __nv_bfloat16_raw*
   A.h = h;
   A.w = w;
   A.part = part;
+  A.flags = flags;
   static bool attr = false;
   if (!attr) {
     if (cudaFuncSetAttribute(k_field_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem) !=

@@ -33,6 +33,7 @@ from .ray import GaussianRay
 from .run import _check_model, _device, pack_model, param_gradients
 
 FIELD_DIRECT, FIELD_SEPARABLE, FIELD_DIRECT_F64 = 0, 1, 2
+_TOO_LARGE = -5  # TG_ERR_TOO_LARGE
 _METHODS = {"direct": FIELD_DIRECT, "separable": FIELD_SEPARABLE, "fp64": FIELD_DIRECT_F64}
 EW_NONSEPARABLE = 0x10
 
@@ -56,6 +57,8 @@ N.register("tg_field_prep_input", C.c_int, [C.POINTER(TgBeams), C.POINTER(TgPixe
                                             C.c_size_t, C.c_void_p, C.c_void_p])
 N.register("tg_decompose_q_inv", C.c_int, [C.c_int64, C.c_void_p, C.c_void_p, C.c_double, C.c_double,
                                            C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p])
+N.register("tg_field_eval_auto", C.c_int, [C.c_int64, C.POINTER(TgPixelMap), C.c_void_p, C.c_void_p,
+                                           C.c_void_p, C.c_size_t, C.c_void_p])
 N.register("tg_field_eval", C.c_int, [C.c_int32, C.c_int64, C.POINTER(TgPixelMap), C.c_void_p,
                                       C.c_void_p, C.c_size_t, C.c_void_p])
 
@@ -205,7 +208,8 @@ class FieldPlan:
     gaussian.py:225-273); or ``model=None`` with ``grid=`` for the field of
     the beams in their own plane (gaussian.py:372-427)."""
 
-    def __init__(self, gaussian_rays: GaussianRay, model, method: str = "auto", *, grid=None):
+    def __init__(self, gaussian_rays: GaussianRay, model, method: str = "auto", *, grid=None,
+                 _settle: bool = True):
         if not isinstance(gaussian_rays, GaussianRay):
             raise TypeError("gaussian_rays must be a GaussianRay (gaussian.py:228)")
         comps = None
@@ -238,17 +242,37 @@ class FieldPlan:
             del keep
             N.check(st, "tg_field_prep")
         if method == "auto":
-            method = "separable" if int(self.flags.item()) == 0 else "direct"
-        if method not in _METHODS:
+            self._method = None
+            if _settle:
+                self.method  # noqa: B018 (read back here: evaluations and captures need not wait)
+        elif method not in _METHODS:
             raise ValueError(f"unknown method {method!r}")
-        self.method = method
+        else:
+            self._method = method
         self.out = torch.empty(self.shape, dtype=torch.complex64, device=self.dev)
         self.comps = comps
         self._vjp_ws = None
 
+    @property
+    def method(self) -> str:
+        """The evaluation's method ("auto" is settled by the preparation's
+        status word)."""
+        if self._method is None:
+            self._method = "separable" if int(self.flags.item()) == 0 else "direct"
+        return self._method
+
     def evaluate(self, method: str | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
-        method = method or self.method
         o = self.out if out is None else out
+        if method is None and self._method is None:
+            # not settled: both methods are launched and the status word picks
+            # one on the device, without waiting for the preparation
+            st = N.lib().tg_field_eval_auto(self.beams.n, C.byref(self.pm), self.flags.data_ptr(),
+                                            torch.view_as_real(o).data_ptr(), self.ws_ptr, self.ws_bytes,
+                                            N.stream_ptr())
+            if st != _TOO_LARGE:  # sizes that the separable method does not take: settled below
+                N.check(st, "tg_field_eval_auto")
+                return o
+        method = method or self.method
         st = N.lib().tg_field_eval(_METHODS[method], self.beams.n, C.byref(self.pm),
                                    torch.view_as_real(o).data_ptr(), self.ws_ptr, self.ws_bytes,
                                    N.stream_ptr())
@@ -365,7 +389,7 @@ def make_gaussian_image(gaussian_rays: GaussianRay, model, batch_size: int = 128
     out = _field_autograd(gaussian_rays, model, method)
     if out is not None:
         return out
-    return FieldPlan(gaussian_rays, model, method).evaluate()
+    return FieldPlan(gaussian_rays, model, method, _settle=False).evaluate()
 
 
 def evaluate_gaussian_input_image(gaussian_rays: GaussianRay, grid, batch_size: int = 128,
@@ -377,7 +401,7 @@ def evaluate_gaussian_input_image(gaussian_rays: GaussianRay, grid, batch_size: 
     out = _field_autograd(gaussian_rays, None, method, grid=grid)
     if out is not None:
         return out
-    return FieldPlan(gaussian_rays, None, method, grid=grid).evaluate()
+    return FieldPlan(gaussian_rays, None, method, grid=grid, _settle=False).evaluate()
 
 
 def decompose_Q_inv(Q_inv, wavelength, eps: float = 1e-12):
