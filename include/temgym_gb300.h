@@ -712,6 +712,11 @@ size_t tg_field_vjp_workspace_ex(int32_t method, int64_t n_beams, int32_t h, int
 int tg_field_vjp_ex(int32_t method, const tg_model *model, const tg_beams *beams, const tg_pixel_map *pm,
                     const float *grad, const tg_field_grads *out, void *workspace, size_t ws_bytes,
                     void *stream);
+/* tg_field_vjp_ex that forms only the entries of out->raw whose byte in
+ * want [2 * n_components][4] (host; NULL = all) is not 0; the others are 0. */
+int tg_field_vjp_steps(int32_t method, const tg_model *model, const tg_beams *beams, const tg_pixel_map *pm,
+                       const float *grad, const tg_field_grads *out, const unsigned char *want,
+                       void *workspace, size_t ws_bytes, void *stream);
 int tg_field_vjp_input_ex(int32_t method, const tg_beams *beams, const tg_pixel_map *pm, const float *grad,
                           const tg_field_grads *out, void *workspace, size_t ws_bytes, void *stream);
 

@@ -34,6 +34,7 @@
 // Every reduction runs in a fixed order, so the gradients are deterministic.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -354,6 +355,41 @@ __device__ __forceinline__ M2<N> operator*(const M2<0>& x, const M2<N>& y) {
   return M2<N>{x.a * y.a + x.b * y.c, x.a * y.b + x.b * y.d, x.c * y.a + x.d * y.c, x.c * y.b + x.d * y.d};
 }
 
+// Real factors (the model's matrices, the rays, the pixel map): a real dual times
+// a complex one is two products instead of four and no zero sums.
+template <int N, typename = std::enable_if_t<(N > 0)>>
+__device__ __forceinline__ Cx<N> operator*(const Du<N>& s, const Cx<0>& a) { return Cx<N>{s * a.re, s * a.im}; }
+template <int N>
+struct R2 {
+  Du<N> a, b, c, d;  // real [[a, b], [c, d]]
+};
+template <int N>
+__device__ __forceinline__ R2<N> operator*(const R2<N>& x, const R2<N>& y) {
+  return R2<N>{x.a * y.a + x.b * y.c, x.a * y.b + x.b * y.d, x.c * y.a + x.d * y.c, x.c * y.b + x.d * y.d};
+}
+template <int N, int K>
+__device__ __forceinline__ M2<N> operator*(const R2<N>& x, const M2<K>& y) {
+  return M2<N>{x.a * y.a + x.b * y.c, x.a * y.b + x.b * y.d, x.c * y.a + x.d * y.c, x.c * y.b + x.d * y.d};
+}
+template <int N>
+__device__ __forceinline__ M2<N> operator+(const R2<N>& x, const M2<N>& y) {
+  return M2<N>{Cx<N>{x.a + y.a.re, y.a.im}, Cx<N>{x.b + y.b.re, y.b.im}, Cx<N>{x.c + y.c.re, y.c.im},
+               Cx<N>{x.d + y.d.re, y.d.im}};
+}
+// nan0(inv2(m)) of a real matrix.  1 / det as det / det^2: non-finite, and so
+// zero, for the determinants (below 1e-154) where the complex quotient is.
+template <int N>
+__device__ __forceinline__ R2<N> inv2_nan0(const R2<N>& m) {
+  const Du<N> det = m.a * m.d - m.b * m.c;
+  const double i2 = 1.0 / (det.v * det.v);
+  if (!isfinite(i2 * det.v)) return R2<N>{dc_<N>(0.0), dc_<N>(0.0), dc_<N>(0.0), dc_<N>(0.0)};
+  Du<N> r;
+  r.v = i2 * det.v;
+#pragma unroll
+  for (int i = 0; i < N; ++i) r.d[i] = -det.d[i] * i2;
+  return R2<N>{fin0(m.d * r), fin0((-1.0) * (m.b * r)), fin0((-1.0) * (m.c * r)), fin0(m.a * r)};
+}
+
 // ------------------------------------------------------------ beam gradient
 // Direction groups, 64 threads a block.  Measured on the separable
 // 16,384-beam adjoint (whole call; Lens + Detector: the central ray's four
@@ -369,7 +405,10 @@ __device__ __forceinline__ M2<N> operator*(const M2<0>& x, const M2<N>& y) {
 // kernel takes 254 registers, so an SM holds 8 of its warps, and it keeps
 // the float64 pipe ~86 % busy; dual and complex divisions by one float64
 // reciprocal (1 divide instead of N + 1, or 2 (N + 1) for a complex
-// quotient) 0.65 -> 0.64 ms.
+// quotient) 0.65 -> 0.64 ms.  The model's matrices and the rays as real factors
+// (two products instead of four and no zero sums) and only the directions that
+// are asked for: at 8,192 beams through Lens + Detector all seven directions
+// 117 -> 92 us, x, y and the focal length alone 51 us.
 constexpr int kBGThreads = 64;
 constexpr int kBGDirs = 4;          // directions a thread carries (at most)
 constexpr int kBGRayDirs = 4;       // central-ray directions a thread carries
@@ -500,14 +539,12 @@ __device__ __forceinline__ void beam_grad_step(const DModel& M, const BGArgs& A,
         break;
     }
   }
-  const M2<ND> Am{cx_<ND>(m[0][0]), cx_<ND>(m[0][1]), cx_<ND>(m[1][0]), cx_<ND>(m[1][1])};
-  const M2<ND> Bm{cx_<ND>(m[0][2]), cx_<ND>(m[0][3]), cx_<ND>(m[1][2]), cx_<ND>(m[1][3])};
-  const M2<ND> Cm{cx_<ND>(m[2][0]), cx_<ND>(m[2][1]), cx_<ND>(m[3][0]), cx_<ND>(m[3][1])};
-  const M2<ND> Dm{cx_<ND>(m[2][2]), cx_<ND>(m[2][3]), cx_<ND>(m[3][2]), cx_<ND>(m[3][3])};
+  const R2<ND> Am{m[0][0], m[0][1], m[1][0], m[1][1]}, Bm{m[0][2], m[0][3], m[1][2], m[1][3]};
+  const R2<ND> Cm{m[2][0], m[2][1], m[3][0], m[3][1]}, Dm{m[2][2], m[2][3], m[3][2], m[3][3]};
   // Q2^-1 = (A + B Q1^-1)^-1 (C + D Q1^-1)   (gaussian.py:92-96)
   const M2<ND> denom = Am + Bm * Q1i;
   const M2<ND> Q2 = inv2(denom) * (Cm + Dm * Q1i);
-  const M2<ND> Binv = nan0(inv2(Bm));
+  const R2<ND> Binv = inv2_nan0(Bm);
   const M2<0> Q1 = nan0(inv2(Q1i));
   const D r2mx = x0 * m[0][0] + y0 * m[0][1] + dx0 * m[0][2] + dy0 * m[0][3];
   const D r2my = x0 * m[1][0] + y0 * m[1][1] + dx0 * m[1][2] + dy0 * m[1][3];
@@ -521,22 +558,20 @@ __device__ __forceinline__ void beam_grad_step(const DModel& M, const BGArgs& A,
     dd.im.v = 0.0;
     dlp = (-0.5) * (dd / cx_<ND>(det.re.v, det.im.v));
   }
-  const M2<ND> ABinv = Am * Binv;
-  const M2<ND> P = Q1 * inv2(Bm * (Am * Q1 + Bm));
+  const R2<ND> ABinv = Am * Binv;
+  const M2<ND> P = Q1 * inv2(Bm * (Bm + Am * Q1));
   Sxx = Q2.a;
   Syy = Q2.d;
   Sxy = 0.5 * (Q2.b + Q2.c);
-  const X bx = x0 * Binv.a + y0 * Binv.c;
-  const X by = x0 * Binv.b + y0 * Binv.d;
-  const X px = P.a * cx_<ND>(r2mx) + P.c * cx_<ND>(r2my);
-  const X py = P.b * cx_<ND>(r2mx) + P.d * cx_<ND>(r2my);
-  Lx = 2.0 * (cx_<ND>(m[2][4]) - bx + px);
-  Ly = 2.0 * (cx_<ND>(m[3][4]) - by + py);
-  const X q1 = x0 * (x0 * ABinv.a + y0 * ABinv.b) +
-               y0 * (x0 * ABinv.c + y0 * ABinv.d);
-  const X q2 = cx_<ND>(r2mx) * (P.a * cx_<ND>(r2mx) + P.b * cx_<ND>(r2my)) +
-               cx_<ND>(r2my) * (P.c * cx_<ND>(r2mx) + P.d * cx_<ND>(r2my));
-  c0 = q1 - q2;
+  const D bx = x0 * Binv.a + y0 * Binv.c;
+  const D by = x0 * Binv.b + y0 * Binv.d;
+  const X px = r2mx * P.a + r2my * P.c;
+  const X py = r2mx * P.b + r2my * P.d;
+  Lx = 2.0 * X{m[2][4] - bx + px.re, px.im};
+  Ly = 2.0 * X{m[3][4] - by + py.re, py.im};
+  const D q1 = x0 * (x0 * ABinv.a + y0 * ABinv.b) + y0 * (x0 * ABinv.c + y0 * ABinv.d);
+  const X q2 = r2mx * (r2mx * P.a + r2my * P.b) + r2my * (r2mx * P.c + r2my * P.d);
+  c0 = X{q1 - q2.re, (-1.0) * q2.im};
   ox = m[0][4];
   oy = m[1][4];
   // the polynomial in (row, col): s = s0 + row u + col v
@@ -609,9 +644,7 @@ __device__ __forceinline__ void beam_grad_step(const DModel& M, const BGArgs& A,
 // ray coordinate are written out (float64, no dual numbers), which is about
 // a third of the float64 work of carrying four dual directions through the
 // whole polynomial.
-template <int NC>
-__device__ __forceinline__ void beam_grad_ray(const DModel& M, const BGArgs& A, int64_t b, int g0, int nd,
-                                              double (&contrib)[NC]) {
+__device__ __forceinline__ void beam_grad_ray(const DModel& M, const BGArgs& A, int64_t b, int g0, int nd) {
   using XP = Cx<0>;
   auto cr = [](double v) { return cx_<0>(v, 0.0); };
   const double x0 = A.x[b], y0 = A.y[b], dx0 = A.dx[b], dy0 = A.dy[b];
@@ -699,36 +732,43 @@ __device__ __forceinline__ void beam_grad_ray(const DModel& M, const BGArgs& A, 
           break;
       }
     }
-    const M2<0> Am{cr(m[0][0]), cr(m[0][1]), cr(m[1][0]), cr(m[1][1])};
-    const M2<0> Bm{cr(m[0][2]), cr(m[0][3]), cr(m[1][2]), cr(m[1][3])};
-    const M2<0> Cm{cr(m[2][0]), cr(m[2][1]), cr(m[3][0]), cr(m[3][1])};
-    const M2<0> Dm{cr(m[2][2]), cr(m[2][3]), cr(m[3][2]), cr(m[3][3])};
+    auto rd = [](double v) { return dc_<0>(v); };
+    const R2<0> Am{rd(m[0][0]), rd(m[0][1]), rd(m[1][0]), rd(m[1][1])};
+    const R2<0> Bm{rd(m[0][2]), rd(m[0][3]), rd(m[1][2]), rd(m[1][3])};
+    const R2<0> Cm{rd(m[2][0]), rd(m[2][1]), rd(m[3][0]), rd(m[3][1])};
+    const R2<0> Dm{rd(m[2][2]), rd(m[2][3]), rd(m[3][2]), rd(m[3][3])};
     const M2<0> Q2 = inv2(Am + Bm * Q1i) * (Cm + Dm * Q1i);
-    const M2<0> Binv = nan0(inv2(Bm));
+    const R2<0> Binv = inv2_nan0(Bm);
     const M2<0> Q1 = nan0(inv2(Q1i));
-    const M2<0> AB = Am * Binv;
-    const M2<0> P = Q1 * inv2(Bm * (Am * Q1 + Bm));
+    const R2<0> AB = Am * Binv;
+    const M2<0> P = Q1 * inv2(Bm * (Bm + Am * Q1));
     Sxx = Q2.a;
     Syy = Q2.d;
     Sxy = 0.5 * (Q2.b + Q2.c);
     const double r2mx = m[0][0] * x0 + m[0][1] * y0 + m[0][2] * dx0 + m[0][3] * dy0;
     const double r2my = m[1][0] * x0 + m[1][1] * y0 + m[1][2] * dx0 + m[1][3] * dy0;
-    const XP abx = AB.a * cr(x0) + AB.b * cr(y0), aby = AB.c * cr(x0) + AB.d * cr(y0);
-    const XP pmx = P.a * cr(r2mx) + P.b * cr(r2my), pmy = P.c * cr(r2mx) + P.d * cr(r2my);
+    const double abx = AB.a.v * x0 + AB.b.v * y0, aby = AB.c.v * x0 + AB.d.v * y0;
+    const XP pmx = r2mx * P.a + r2my * P.b, pmy = r2mx * P.c + r2my * P.d;
+#pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const double ex = c == 0 ? 1.0 : 0.0, ey = c == 1 ? 1.0 : 0.0;  // d (x0, y0)
-      const double erx = m[0][c], ery = m[1][c];                      // d (r2mx, r2my)
+      const double erx = m[0][c], ery = m[1][c];  // d (r2mx, r2my); d (x0, y0) is (1, 0), (0, 1), 0, 0
       // L = 2 (m[2..3][4] - B^-1^T r1m + P^T r2m): the first part is constant
-      const XP dbx = Binv.a * cr(ex) + Binv.c * cr(ey), dby = Binv.b * cr(ex) + Binv.d * cr(ey);
-      const XP dpx = P.a * cr(erx) + P.c * cr(ery), dpy = P.b * cr(erx) + P.d * cr(ery);
-      dLx[c] = 2.0 * (dpx - dbx);
-      dLy[c] = 2.0 * (dpy - dby);
+      XP dpx = erx * P.a + ery * P.c, dpy = erx * P.b + ery * P.d;
       // c0 = r1m^T (A B^-1) r1m - r2m^T P r2m
-      const XP dq1 = cr(ex) * abx + cr(x0) * (AB.a * cr(ex) + AB.b * cr(ey)) + cr(ey) * aby +
-                     cr(y0) * (AB.c * cr(ex) + AB.d * cr(ey));
-      const XP dq2 = cr(erx) * pmx + cr(r2mx) * (P.a * cr(erx) + P.b * cr(ery)) + cr(ery) * pmy +
-                     cr(r2my) * (P.c * cr(erx) + P.d * cr(ery));
-      dc0[c] = dq1 - dq2;
+      const XP dq2 = erx * pmx + r2mx * (erx * P.a + ery * P.b) + ery * pmy + r2my * (erx * P.c + ery * P.d);
+      double dq1 = 0.0;
+      if (c == 0) {
+        dpx.re.v -= Binv.a.v;
+        dpy.re.v -= Binv.b.v;
+        dq1 = abx + x0 * AB.a.v + y0 * AB.c.v;
+      } else if (c == 1) {
+        dpx.re.v -= Binv.c.v;
+        dpy.re.v -= Binv.d.v;
+        dq1 = x0 * AB.b.v + aby + y0 * AB.d.v;
+      }
+      dLx[c] = 2.0 * dpx;
+      dLy[c] = 2.0 * dpy;
+      dc0[c] = cx_<0>(dq1 - dq2.re.v, -dq2.im.v);
       ds0x[c] = 0.0;
       ds0y[c] = 0.0;
     }
@@ -754,21 +794,27 @@ __device__ __forceinline__ void beam_grad_ray(const DModel& M, const BGArgs& A, 
   const double wr5 = ar * ur5 - ai * ui5, wi5 = ar * ui5 + ai * ur5;
   // dL/dp = -sum_j Im(dkap_j w_j) over j = col, row, 1 (kap_cc, kap_rr,
   // kap_rc and the prefactor do not move with the central ray)
-  for (int d = 0; d < nd && d < NC; ++d) {
-    const int kd = A.dir_kind[g0 + d];
-    if (kd < DIR_X || kd > DIR_DY) continue;
-    const int c = kd;  // DIR_X .. DIR_DY = 0 .. 3
-    const XP k3 = hk * (2.0 * quad(ds0x[c], ds0y[c], vx, vy) + vx * dLx[c] + vy * dLy[c]);
-    const XP k4 = hk * (2.0 * quad(ds0x[c], ds0y[c], ux, uy) + ux * dLx[c] + uy * dLy[c]);
-    const XP k5 = hk * (2.0 * quad(ds0x[c], ds0y[c], s0x, s0y) + ds0x[c] * Lx + ds0y[c] * Ly + s0x * dLx[c] +
-                        s0y * dLy[c] + dc0[c]);
-    const double g = -(k3.re.v * wi3 + k3.im.v * wr3) - (k4.re.v * wi4 + k4.im.v * wr4) -
-                     (k5.re.v * wi5 + k5.im.v * wr5);
-    contrib[d] = g;
-    if (kd == DIR_X && A.gx) A.gx[b] = g;
-    if (kd == DIR_Y && A.gy) A.gy[b] = g;
-    if (kd == DIR_DX && A.gdx) A.gdx[b] = g;
-    if (kd == DIR_DY && A.gdy) A.gdy[b] = g;
+  // the curvatures do not move with the ray, but a beam without finite ones has
+  // no gradient: 0 times them (NaN then) goes into each
+  double none = 0.0;
+  for (const XP* q : {&Sxx, &Syy, &Sxy}) none = fma(0.0, q->re.v, fma(0.0, q->im.v, none));
+  int want = 0;  // the same for the whole launch
+  for (int d = 0; d < nd; ++d)
+    if (A.dir_kind[g0 + d] <= DIR_DY) want |= 1 << A.dir_kind[g0 + d];
+#pragma unroll
+  for (int c = DIR_X; c <= DIR_DY; ++c) {
+    if (!(want >> c & 1)) continue;
+    XP k3 = vx * dLx[c] + vy * dLy[c], k4 = ux * dLx[c] + uy * dLy[c];
+    XP k5 = s0x * dLx[c] + s0y * dLy[c] + dc0[c];
+    if (A.input_plane) {  // s0 moves with x and y only there
+      k3 = 2.0 * quad(ds0x[c], ds0y[c], vx, vy) + k3;
+      k4 = 2.0 * quad(ds0x[c], ds0y[c], ux, uy) + k4;
+      k5 = 2.0 * quad(ds0x[c], ds0y[c], s0x, s0y) + ds0x[c] * Lx + ds0y[c] * Ly + k5;
+    }
+    const double g = -hk * ((k3.re.v * wi3 + k3.im.v * wr3) + (k4.re.v * wi4 + k4.im.v * wr4) +
+                            (k5.re.v * wi5 + k5.im.v * wr5)) + none;
+    double* const to = c == DIR_X ? A.gx : c == DIR_Y ? A.gy : c == DIR_DX ? A.gdx : A.gdy;
+    if (to) to[b] = g;
   }
   if (A.gpl && blockIdx.y == 0) A.gpl[b] = -k * wi5;
   if (A.gamp && blockIdx.y == 0) {
@@ -815,7 +861,7 @@ k_field_beam_grad(const __grid_constant__ DModel M, const __grid_constant__ BGAr
     if (step)
       beam_grad_fit<kBGStepDirs>(M, A, b, g0, nd, contrib);
     else
-      beam_grad_ray(M, A, b, g0, nd, contrib);
+      beam_grad_ray(M, A, b, g0, nd);
   }
   // the block's sums of the model directions, in a fixed order
 #pragma unroll
@@ -1077,7 +1123,7 @@ int launch_field_gemm(const __nv_bfloat16_raw* vplanes, const __nv_bfloat16_raw*
 
 static int field_vjp_impl(const tg_model* model, const tg_beams* beams, const tg_pixel_map* pm,
                           const float* grad, const tg_field_grads* out, void* workspace, size_t ws_bytes,
-                          void* stream, int method = TG_FIELD_DIRECT) {
+                          void* stream, int method = TG_FIELD_DIRECT, const unsigned char* want = nullptr) {
   if (method != TG_FIELD_DIRECT && method != TG_FIELD_SEPARABLE) return TG_ERR_INVALID;
   if (!beams || !pm || !grad || !out || pm->h <= 0 || pm->w <= 0 || beams->n < 0) return TG_ERR_INVALID;
   const bool input_plane = model == nullptr;
@@ -1139,10 +1185,10 @@ static int field_vjp_impl(const tg_model* model, const tg_beams* beams, const tg
   }
   // 3. directions: the central ray's x, y, dx, dy, then the model's step parameters
   std::vector<Dir> dirs;
-  const bool ray = out->x || out->y || out->dx || out->dy;
-  if (ray) {
-    for (int j = 0; j < 4; ++j) dirs.push_back(Dir{j, 0, 0, 1.0, -1});
-  }
+  // (those asked for: each costs a pass through its group's algebra)
+  const double* const ray[4] = {out->x, out->y, out->dx, out->dy};
+  for (int j = 0; j < 4; ++j)
+    if (ray[j]) dirs.push_back(Dir{j, 0, 0, 1.0, -1});
   if (out->raw) {
     for (int s2 = 0; s2 < dm.n; ++s2) {
       const DStep& stp = dm.s[s2];
@@ -1163,6 +1209,9 @@ static int field_vjp_impl(const tg_model* model, const tg_beams* beams, const tg
         default: break;
       }
     }
+    if (want)
+      dirs.erase(std::remove_if(dirs.begin(), dirs.end(), [&](const Dir& d) { return d.target >= 0 && !want[d.target]; }),
+                 dirs.end());
   }
   double* mpart = reinterpret_cast<double*>(ws + L.model);
   // launches of up to kBGLaunchDirs directions, kBGDirs a thread (groups on blockIdx.y)
@@ -1254,6 +1303,13 @@ extern "C" int tg_field_vjp_ex(int32_t method, const tg_model* model, const tg_b
                                void* workspace, size_t ws_bytes, void* stream) {
   if (!model) return TG_ERR_INVALID;
   return field_vjp_impl(model, beams, pm, grad, out, workspace, ws_bytes, stream, method);
+}
+
+extern "C" int tg_field_vjp_steps(int32_t method, const tg_model* model, const tg_beams* beams, const tg_pixel_map* pm,
+                                  const float* grad, const tg_field_grads* out, const unsigned char* want,
+                                  void* workspace, size_t ws_bytes, void* stream) {
+  if (!model) return TG_ERR_INVALID;
+  return field_vjp_impl(model, beams, pm, grad, out, workspace, ws_bytes, stream, method, want);
 }
 
 extern "C" int tg_field_vjp_input_ex(int32_t method, const tg_beams* beams, const tg_pixel_map* pm,

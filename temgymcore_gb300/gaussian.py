@@ -30,7 +30,7 @@ import torch
 from . import _native as N
 from .components import Grid
 from .ray import GaussianRay
-from .run import _check_model, _device, pack_model, param_gradients
+from .run import _check_model, _device, pack_model, param_gradients, param_steps
 
 FIELD_DIRECT, FIELD_SEPARABLE, FIELD_DIRECT_F64 = 0, 1, 2
 _TOO_LARGE = -5  # TG_ERR_TOO_LARGE
@@ -77,6 +77,9 @@ N.register("tg_field_vjp_workspace_ex", C.c_size_t, [C.c_int32, C.c_int64, C.c_i
 N.register("tg_field_vjp_ex", C.c_int, [C.c_int32, C.POINTER(N.TgModel), C.POINTER(TgBeams),
                                         C.POINTER(TgPixelMap), C.c_void_p, C.POINTER(TgFieldGrads),
                                         C.c_void_p, C.c_size_t, C.c_void_p])
+N.register("tg_field_vjp_steps", C.c_int, [C.c_int32, C.POINTER(N.TgModel), C.POINTER(TgBeams),
+                                           C.POINTER(TgPixelMap), C.c_void_p, C.POINTER(TgFieldGrads),
+                                           C.c_char_p, C.c_void_p, C.c_size_t, C.c_void_p])
 N.register("tg_field_vjp_input_ex", C.c_int, [C.c_int32, C.POINTER(TgBeams), C.POINTER(TgPixelMap), C.c_void_p,
                                               C.POINTER(TgFieldGrads), C.c_void_p, C.c_size_t, C.c_void_p])
 
@@ -201,6 +204,9 @@ class BeamSet:
         return b
 
 
+_BEAM_FIELDS = ("amplitude", "pathlength", "x", "y", "dx", "dy")
+
+
 class FieldPlan:
     """Prepared beams + workspace for repeated field evaluations.
 
@@ -283,7 +289,8 @@ class FieldPlan:
     def separable(self) -> bool:
         return int(self.flags.item()) == 0
 
-    def vjp(self, grad: torch.Tensor, beams: bool = True, model: bool = True, method: str | None = None) -> dict:
+    def vjp(self, grad: torch.Tensor, beams: bool = True, model: bool = True, method: str | None = None,
+            *, _fields=_BEAM_FIELDS, _steps: bytes | None = None) -> dict:
         """Gradients of a real loss L from its gradient with respect to the
         field, ``grad`` = dL/dRe F + i dL/dIm F (complex (H, W), PyTorch's
         convention): per beam ``amplitude`` (complex64), ``pathlength``,
@@ -305,10 +312,8 @@ class FieldPlan:
         res = {}
         out = TgFieldGrads()
         if beams:
-            res["amplitude"] = torch.empty(n, dtype=torch.complex64, device=dev)
-            out.amplitude = torch.view_as_real(res["amplitude"]).data_ptr()
-            for k in ("pathlength", "x", "y", "dx", "dy"):
-                res[k] = torch.empty(n, dtype=torch.float64, device=dev)
+            for k in _fields:
+                res[k] = torch.empty(n, dtype=torch.complex64 if k == "amplitude" else torch.float64, device=dev)
                 setattr(out, k, res[k].data_ptr())
         if model and self.comps is not None:
             res["raw"] = torch.empty((2 * len(self.comps), 4), dtype=torch.float64, device=dev)
@@ -320,15 +325,12 @@ class FieldPlan:
             N.check(st, "tg_field_vjp_input_ex")
         else:
             m, keep = pack_model(self.comps)
-            st = N.lib().tg_field_vjp_ex(code, C.byref(m), C.byref(self.beams.struct()), C.byref(self.pm),
-                                         g.data_ptr(), C.byref(out), ws.data_ptr() + off, ws.numel() - off,
-                                         N.stream_ptr())
+            st = N.lib().tg_field_vjp_steps(code, C.byref(m), C.byref(self.beams.struct()), C.byref(self.pm),
+                                            g.data_ptr(), C.byref(out), _steps, ws.data_ptr() + off,
+                                            ws.numel() - off, N.stream_ptr())
             del keep
-            N.check(st, "tg_field_vjp_ex")
+            N.check(st, "tg_field_vjp_steps")
         return res
-
-
-_BEAM_FIELDS = ("amplitude", "pathlength", "x", "y", "dx", "dy")
 
 
 class _FieldFn(torch.autograd.Function):
@@ -339,18 +341,18 @@ class _FieldFn(torch.autograd.Function):
     def forward(ctx, spec, *inputs):
         plan = spec["plan"]
         ctx.spec = spec
-        return plan.evaluate(spec["method"])  # the plan's own buffer: nothing else evaluates it
+        return plan.evaluate()  # the plan's own buffer: nothing else evaluates it
 
     @staticmethod
     def backward(ctx, grad):
         spec = ctx.spec
         plan = spec["plan"]
-        r = plan.vjp(grad, beams=bool(spec["beam_inputs"]), model=bool(spec["params"]))
+        params = spec["params"]
+        r = plan.vjp(grad, beams=bool(spec["beam_inputs"]), model=bool(params),
+                     _fields=[name for name, _ in spec["beam_inputs"]],
+                     _steps=param_steps(plan.comps, params) if params else None)
         out = []
         for name, t in spec["beam_inputs"]:
-            if t is None:
-                out.append(None)
-                continue
             g = r[name]
             if t.numel() == 1 and g.numel() != 1:
                 g = g.sum()
@@ -373,8 +375,8 @@ def _field_autograd(gaussian_rays: GaussianRay, model, method: str, grid=None):
     params = _grad_params(_check_model(model)) if model is not None else []
     if not params and all(t is None for _, t in beam_inputs):
         return None
-    plan = FieldPlan(gaussian_rays, model, method, grid=grid)
-    spec = {"plan": plan, "method": plan.method, "beam_inputs": beam_inputs, "params": params}
+    plan = FieldPlan(gaussian_rays, model, method, grid=grid, _settle=False)
+    spec = {"plan": plan, "beam_inputs": beam_inputs, "params": params}
     tensors = [t for _, t in beam_inputs if t is not None] + [t for (_, _, t) in params]
     spec["beam_inputs"] = [(n_, t) for n_, t in beam_inputs if t is not None]
     return _FieldFn.apply(spec, *tensors)

@@ -181,7 +181,6 @@ def param_gradient(comps, i, path, raw):
     (a float64 tensor, or a NumPy array of the sums read back to the host)."""
     c = comps[i]
     nc = len(comps)
-    comp = raw[2 * i + 1]
     if path in ("z", "z_po"):
         g = raw[2 * i, 0]
         if i + 1 < nc and not isinstance(c, ThickLens):
@@ -189,6 +188,7 @@ def param_gradient(comps, i, path, raw):
         return g
     if path == "z_pi":
         return -raw[2 * i + 2, 0] if i + 1 < nc else raw[0, 0] * 0.0
+    comp = raw[2 * i + 1]
     if path == "focal_length" or path == "def_x":
         return comp[0]
     if path == "def_y":
@@ -229,6 +229,27 @@ def param_gradients(comps, plist, raw) -> list:
             g = torch.tensor(float(param_gradient(comps, i, path, host)), dtype=t.dtype)
             out.append(g if t.dim() == 0 else g.reshape(t.shape))
     return out
+
+
+class _SumsRead:
+    """Stands in for the per-step sums and notes the entries that are read."""
+
+    def __init__(self, nc: int):
+        self.want = np.zeros((2 * nc, 4), dtype=np.uint8)
+        self.zeros = np.zeros((2 * nc, 4))
+
+    def __getitem__(self, key):
+        self.want[key] = 1
+        return self.zeros[key]
+
+
+def param_steps(comps, plist) -> bytes:
+    """Which of the per-step sums [(2 * n_components), 4] the gradients of
+    ``plist`` (_grad_params) read: one byte each, 1 = read."""
+    rec = _SumsRead(len(comps))
+    for i, path, _ in plist:
+        param_gradient(comps, i, path, rec)
+    return rec.want.tobytes()
 
 
 class _TraceFn(torch.autograd.Function):
