@@ -174,17 +174,179 @@ __device__ void batch_model_tail(const BModel& M, int model, const double* parti
   if (loss && threadIdx.x == 0) loss[model] = mo[kMomLoss];
 }
 
+// The rays [it, it + R blockDim) of a tile (x, y, dx, dy and the targets) arrive by
+// cp.async while the rays before them are traced: 4-byte copies into this thread's
+// own slots of stage st, no barrier.
+template <int R>
+__device__ __forceinline__ void batch_prefetch(const BatchIO& io, const BTile& T, uint32_t pf_base, int nf, bool adj,
+                                               int it, int st) {
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    const int id = it + (int)threadIdx.x + k * (int)blockDim.x;
+    const uint32_t sz = id < T.count ? 4u : 0u;
+    const int64_t g = T.start + (id < T.count ? id : 0);
+    const uint32_t b = pf_base + 4u * (uint32_t)((st * nf * R + k) * (int)blockDim.x + (int)threadIdx.x);
+    const uint32_t fs = 4u * (uint32_t)(R * (int)blockDim.x);
+    cp_async4(b + 0 * fs, io.x + g, sz);
+    cp_async4(b + 1 * fs, io.y + g, sz);
+    cp_async4(b + 2 * fs, io.dx + g, sz);
+    cp_async4(b + 3 * fs, io.dy + g, sz);
+    if (adj) {
+      cp_async4(b + 4 * fs, io.tx + g, sz);
+      cp_async4(b + 5 * fs, io.ty + g, sz);
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// Whether a tile runs two rays at a time: always where a thread has two and the
+// signs fit registers (256 threads x 2 rays, 512 models: 323 us, 340 one by one;
+// up to two biprisms only: 327).  Bound by instructions issued and the shared
+// memory reads of the records, at half occupancy (64 registers; 3 blocks of 80: 343).
+constexpr bool batch_pairs(int R, int nb) { return R >= 2 && nb >= 0; }
+
+// Two rays of a tile at a time (R >= 2, at most four biprisms), as batch_tile
+// forms each: the rays are the halves of packed pairs, the record is held twice
+// over in shared memory (srec2: every float as a pair), so that one 16-byte read
+// brings two coefficients for both rays.  The moments are added ray by ray, in
+// batch_tile's order: the same sums.
+template <int R, int NB>
+__device__ __forceinline__ void batch_pair(const BatchIO& io, const BModel& M, const F2* srec2,
+                                           const float* pb, int fsf, int64_t t0, int idx0, int cnt, bool adj,
+                                           float (&mw)[11], float (&bsx)[NB > 0 ? NB : 1], float (&bsy)[NB > 0 ? NB : 1]) {
+  constexpr int NS = NB > 0 ? NB : 1;
+  const RecLayout L = rec_layout(NB, 0, 0);
+  const int bd = (int)blockDim.x;
+  F2 v[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) v[c] = f2(pb[c * fsf], pb[c * fsf + bd]);
+  F2 sg[NS];
+#pragma unroll
+  for (int b = 0; b < NS; ++b) sg[b] = F2{0ull};
+  bool alive0 = true, alive1 = true;
+  auto two = [](const F2* q) { return *reinterpret_cast<const ulonglong2*>(q); };
+  auto dot = [&](const F2* row) {
+    const ulonglong2 r0 = two(row), r1 = two(row + 2), r2 = two(row + 4);
+    F2 acc = f2_fma(F2{r0.x}, v[0], F2{r2.x});
+    acc = f2_fma(F2{r0.y}, v[1], acc);
+    acc = f2_fma(F2{r1.x}, v[2], acc);
+    acc = f2_fma(F2{r1.y}, v[3], acc);
+    if (NB > 0) acc = f2_fma(F2{r2.y}, sg[0], acc);
+#pragma unroll
+    for (int b = 1; b < NB; ++b) acc = f2_fma(row[5 + b], sg[b < NS ? b : 0], acc);
+    return acc;
+  };
+  {
+    const F2* e = srec2 + M.ev_off;
+    int nbs = 0;
+    for (int qe = 0; qe < M.n_ev; ++qe) {
+      if (__float_as_int(f2_lo(e[0])) == kEvBiprism) {
+        const F2 xe = dot(e + 8);
+        const float x0 = f2_lo(xe), x1 = f2_hi(xe);
+        const F2 s = f2(x0 > 0.f ? 1.f : (x0 < 0.f ? -1.f : 0.f), x1 > 0.f ? 1.f : (x1 < 0.f ? -1.f : 0.f));
+#pragma unroll
+        for (int b = 0; b < NS; ++b)
+          if (b == nbs) sg[b] = s;
+        ++nbs;
+        e += 8 + L.D4;
+      } else {
+        const F2 ex = dot(e + 8), ey = dot(e + 8 + L.D4);
+        const F2 d = f2_fma(ex, ex, f2_mul(ey, ey));
+        const float r2 = f2_lo(e[2]);
+        alive0 = alive0 && f2_lo(d) < r2;
+        alive1 = alive1 && f2_hi(d) < r2;
+        e += 8 + 2 * L.D4;
+      }
+    }
+  }
+  ulonglong2 lo = two(srec2 + 16), hi = two(srec2 + 18);
+  F2 a0{lo.x}, a1{lo.y}, a2{hi.x}, a3{hi.y};
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    lo = two(srec2 + 4 * c);
+    hi = two(srec2 + 4 * c + 2);
+    a0 = f2_fma(F2{lo.x}, v[c], a0);
+    a1 = f2_fma(F2{lo.y}, v[c], a1);
+    a2 = f2_fma(F2{hi.x}, v[c], a2);
+    a3 = f2_fma(F2{hi.y}, v[c], a3);
+  }
+  F2 p;
+  {
+    const F2* q = srec2 + L.q;
+    const ulonglong2 q0 = two(q), q2 = two(q + 2), q4 = two(q + 4), q6 = two(q + 6), q8 = two(q + 8), q10 = two(q + 10),
+                     q12 = two(q + 12), q14 = two(q + 14);
+    const F2 t0q = f2_fma(v[3], F2{q8.x}, f2_fma(v[2], F2{q6.y}, f2_fma(v[1], F2{q6.x}, f2_fma(v[0], F2{q4.y}, F2{q0.y}))));
+    const F2 t1q = f2_fma(v[3], F2{q10.y}, f2_fma(v[2], F2{q10.x}, f2_fma(v[1], F2{q8.y}, F2{q2.x})));
+    const F2 t2q = f2_fma(v[3], F2{q12.y}, f2_fma(v[2], F2{q12.x}, F2{q2.y}));
+    const F2 t3q = f2_fma(v[3], F2{q14.x}, F2{q4.x});
+    p = f2_fma(v[0], t0q, f2_fma(v[1], t1q, f2_fma(v[2], t2q, f2_mul(v[3], t3q))));
+  }
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const F2 s = sg[b < NS ? b : 0];
+    lo = two(srec2 + 20 + 4 * b);
+    hi = two(srec2 + 22 + 4 * b);
+    a0 = f2_fma(F2{lo.x}, s, a0);
+    a1 = f2_fma(F2{lo.y}, s, a1);
+    a2 = f2_fma(F2{hi.x}, s, a2);
+    a3 = f2_fma(F2{hi.y}, s, a3);
+    const F2* lb = srec2 + L.l + 8 * b;
+    lo = two(lb);
+    hi = two(lb + 2);
+    F2 lin = f2_fma(F2{lo.x}, v[0], f2_fma(F2{lo.y}, v[1], f2_fma(F2{hi.x}, v[2], f2_fma(F2{hi.y}, v[3], lb[4]))));
+    const F2* kb = srec2 + L.k + b * NB - (b * (b - 1)) / 2;
+#pragma unroll
+    for (int b2 = b; b2 < NB; ++b2) lin = f2_fma(kb[b2 - b], sg[b2 < NS ? b2 : 0], lin);
+    p = f2_fma(s, lin, p);
+  }
+  auto finish = [&](int idx, float o0, float o1, float o2, float o3, float pl, bool alive, const float* tgt, F2 (&vv)[4],
+                    bool second) {
+    const bool inr = idx < cnt;
+    if (inr) {
+      const int64_t i = t0 + idx;
+      io.ox[i] = o0;
+      io.oy[i] = o1;
+      io.odx[i] = o2;
+      io.ody[i] = o3;
+      if (io.opl) io.opl[i] = M.pl_const + (double)pl;
+      if (io.alive) io.alive[i] = alive ? 1 : 0;
+    }
+    if (!adj) return;
+    const bool use = inr && alive;
+    const float rx = use ? o0 - tgt[4 * fsf] : 0.f, ry = use ? o1 - tgt[5 * fsf] : 0.f;
+    const float lx = 2.f * rx, ly = 2.f * ry;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float vc = second ? f2_hi(vv[c]) : f2_lo(vv[c]);
+      mw[c] = fmaf(lx, vc, mw[c]);
+      mw[5 + c] = fmaf(ly, vc, mw[5 + c]);
+    }
+    mw[4] += lx;
+    mw[9] += ly;
+    mw[kMomLoss] = fmaf(rx, rx, fmaf(ry, ry, mw[kMomLoss]));
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const float s = second ? f2_hi(sg[b < NS ? b : 0]) : f2_lo(sg[b < NS ? b : 0]);
+      bsx[b < NS ? b : 0] = fmaf(s, lx, bsx[b < NS ? b : 0]);
+      bsy[b < NS ? b : 0] = fmaf(s, ly, bsy[b < NS ? b : 0]);
+    }
+  };
+  finish(idx0, f2_lo(a0), f2_lo(a1), f2_lo(a2), f2_lo(a3), f2_lo(p), alive0, pb, v, false);
+  finish(idx0 + bd, f2_hi(a0), f2_hi(a1), f2_hi(a2), f2_hi(a3), f2_hi(p), alive1, pb + bd, v, true);
+}
+
 // One tile of one model: every ray of the tile from start to finish (events,
 // outputs, pathlength, stores, moments), then the tile's moments summed per
 // warp into wacc.  NB = the model's biprism count when it is at most four:
 // the signs live in registers and every loop over them is unrolled; NB = -1:
 // any count, signs as bit masks with runtime loops.
 template <int R, int NB>
-__device__ __forceinline__ void batch_tile(const BatchIO& io, const BModel& M, const RecLayout& L,
-                                           const float* srec, const float* pf, uint32_t pf_base,
+__device__ __forceinline__ void batch_tile(const BatchIO& io, const BModel& M, const float* srec, const float* pf, uint32_t pf_base,
                                            const BTile& T, int nf, bool adj, float* wacc) {
   constexpr int NS = NB > 0 ? NB : (NB < 0 ? kRegBip : 1);  // register sign slots
-  const int nb = M.n_bip, nm = M.n_mom;
+  constexpr bool kPair = batch_pairs(R, NB);
+  const int nb = NB >= 0 ? NB : M.n_bip, nm = kMomBip + 2 * nb;
+  const RecLayout L = rec_layout(nb, 0, 0);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t t0 = T.start;
   float mw[11];
@@ -195,30 +357,7 @@ __device__ __forceinline__ void batch_tile(const BatchIO& io, const BModel& M, c
   for (int j = 0; j < NS; ++j) bsx[j] = bsy[j] = 0.f;
   const int cnt = T.count;
   const int per = blockDim.x * R;
-  // the next iteration's x, y, dx, dy (and targets) arrive by cp.async
-  // (4-byte copies into this thread's own slots: no barrier) while this one
-  // computes
-  auto prefetch = [&](int it2, int st2) {
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-      const int id = it2 + (int)threadIdx.x + k * (int)blockDim.x;
-      const uint32_t sz = id < cnt ? 4u : 0u;
-      const int i = id < cnt ? id : 0;
-      const uint32_t b = pf_base + 4u * (uint32_t)((st2 * nf * R + k) * (int)blockDim.x + (int)threadIdx.x);
-      const uint32_t fs = 4u * (uint32_t)(R * (int)blockDim.x);
-      const int64_t g = t0 + i;
-      cp_async4(b + 0 * fs, io.x + g, sz);
-      cp_async4(b + 1 * fs, io.y + g, sz);
-      cp_async4(b + 2 * fs, io.dx + g, sz);
-      cp_async4(b + 3 * fs, io.dy + g, sz);
-      if (adj) {
-        cp_async4(b + 4 * fs, io.tx + g, sz);
-        cp_async4(b + 5 * fs, io.ty + g, sz);
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  prefetch(0, 0);
+  auto prefetch = [&](int it2, int st2) { batch_prefetch<R>(io, T, pf_base, nf, adj, it2, st2); };
   const float4* col = reinterpret_cast<const float4*>(srec);
   const float* q = srec + L.q;
   for (int it = 0, st = 0; it < cnt; it += per, st ^= 1) {
@@ -226,6 +365,14 @@ __device__ __forceinline__ void batch_tile(const BatchIO& io, const BModel& M, c
     else asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     const int fsf = R * (int)blockDim.x;
+    if constexpr (kPair) {
+      float(&bx)[NS] = bsx, (&by)[NS] = bsy;
+#pragma unroll 1
+      for (int k = 0; k < R; k += 2)
+        batch_pair<R, NB>(io, M, reinterpret_cast<const F2*>(srec), pf + (st * nf * R + k) * (int)blockDim.x + (int)threadIdx.x,
+                          fsf, t0, it + (int)threadIdx.x + k * (int)blockDim.x, cnt, adj, mw, bx, by);
+      continue;
+    }
     // one ray at a time from start to finish: only its state is live, and
     // the record's coefficients are re-read from shared memory per ray
 #pragma unroll 1
@@ -437,22 +584,31 @@ k_batch(const uint8_t* __restrict__ plan, const __grid_constant__ BatchIO io,
       continue;
     }
     const int nm = M.n_mom, nb = M.n_bip;
-    const RecLayout L = rec_layout(nb, 0, 0);
+    batch_prefetch<R>(io, T, pf_base, nf, adj, 0, 0);
     {
       const float4* src = reinterpret_cast<const float4*>(recs + M.rec_off);
       float4* dst = reinterpret_cast<float4*>(srec);
-      for (int i = threadIdx.x; i < (M.rec_floats >> 2); i += blockDim.x) dst[i] = __ldg(src + i);
+      const bool twice = batch_pairs(R, nb <= kRegBip ? nb : -1);
+      for (int i = threadIdx.x; i < (M.rec_floats >> 2); i += blockDim.x) {
+        const float4 r = __ldg(src + i);
+        if (twice) {
+          dst[2 * i] = make_float4(r.x, r.x, r.y, r.y);
+          dst[2 * i + 1] = make_float4(r.z, r.z, r.w, r.w);
+        } else {
+          dst[i] = r;
+        }
+      }
     }
     if (adj)
       for (int i = threadIdx.x; i < nwarps * nm; i += blockDim.x) wacc[i] = 0.f;
     __syncthreads();
     switch (nb) {  // signs as registers in fully unrolled loops for up to four biprisms
-      case 0: batch_tile<R, 0>(io, M, L, srec, pf, pf_base, T, nf, adj, wacc); break;
-      case 1: batch_tile<R, 1>(io, M, L, srec, pf, pf_base, T, nf, adj, wacc); break;
-      case 2: batch_tile<R, 2>(io, M, L, srec, pf, pf_base, T, nf, adj, wacc); break;
-      case 3: batch_tile<R, 3>(io, M, L, srec, pf, pf_base, T, nf, adj, wacc); break;
-      case 4: batch_tile<R, 4>(io, M, L, srec, pf, pf_base, T, nf, adj, wacc); break;
-      default: batch_tile<R, -1>(io, M, L, srec, pf, pf_base, T, nf, adj, wacc); break;
+      case 0: batch_tile<R, 0>(io, M, srec, pf, pf_base, T, nf, adj, wacc); break;
+      case 1: batch_tile<R, 1>(io, M, srec, pf, pf_base, T, nf, adj, wacc); break;
+      case 2: batch_tile<R, 2>(io, M, srec, pf, pf_base, T, nf, adj, wacc); break;
+      case 3: batch_tile<R, 3>(io, M, srec, pf, pf_base, T, nf, adj, wacc); break;
+      case 4: batch_tile<R, 4>(io, M, srec, pf, pf_base, T, nf, adj, wacc); break;
+      default: batch_tile<R, -1>(io, M, srec, pf, pf_base, T, nf, adj, wacc); break;
     }
     __syncthreads();
     if (adj) {
@@ -913,7 +1069,7 @@ extern "C" int tg_batch_run(const void* plan_dev, const tg_batch_info* info, con
   if (tail > dyn) dyn = tail;
   dyn = (dyn + 15) & ~(size_t)15;
   const int rec_smem_off = (int)(dyn / sizeof(float));
-  dyn += ((size_t)info->max_record_floats * sizeof(float) + 15) & ~(size_t)15;
+  dyn += ((size_t)info->max_record_floats * (rays_per_thread >= 2 ? 2 : 1) * sizeof(float) + 15) & ~(size_t)15;
   const int pf_off = (int)(dyn / sizeof(float));
   dyn += (size_t)2 * (adj ? 6 : 4) * rays_per_thread * block * sizeof(float);
   if (dyn > 200 * 1024) return TG_ERR_TOO_LARGE;

@@ -93,37 +93,7 @@ __device__ __forceinline__ double df_to_double(float h, float l) {
 }
 
 // ------------------------------------------------- two double-floats at a time
-// Packed pairs of float32 (the component of x and the component of y): one
-// instruction issues both, and each half rounds as the scalar operation does.
-struct F2 {
-  unsigned long long u;
-};
-__device__ __forceinline__ F2 f2(float a, float b) {
-  return F2{((unsigned long long)__float_as_uint(b) << 32) | __float_as_uint(a)};
-}
-__device__ __forceinline__ float f2_lo(F2 a) { return __uint_as_float((uint32_t)a.u); }
-__device__ __forceinline__ float f2_hi(F2 a) { return __uint_as_float((uint32_t)(a.u >> 32)); }
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
-  F2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.u) : "l"(a.u), "l"(b.u));
-  return d;
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-  F2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.u) : "l"(a.u), "l"(b.u), "l"(c.u));
-  return d;
-}
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
-  F2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.u) : "l"(a.u), "l"(b.u));
-  return d;
-}
-__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {
-  F2 d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d.u) : "l"(a.u), "l"(b.u));
-  return d;
-}
-
+// (packed pairs: the component of x and the component of y)
 // A pair of ray components, with the negated parts that the products below use.
 struct Ray2 {
   F2 h, nh, nl;
