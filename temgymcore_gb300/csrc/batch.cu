@@ -978,10 +978,16 @@ extern "C" int tg_batch_plan(int32_t n_models, const tg_model* models, const int
       return TG_ERR_TOO_LARGE;
   }
   {  // longest tiles first (the work counter hands them out in list order), so
-     // the launch ends on small tiles; ties keep model order
+     // the launch ends on small tiles; ties by the biprisms (the code that the
+     // tile runs: neighbours share it in the instruction cache, 323 -> 319 us at
+     // 512 models) and events, then in model order
     std::vector<int32_t> ord(bt.size());
     for (size_t i = 0; i < ord.size(); ++i) ord[i] = (int32_t)i;
-    std::stable_sort(ord.begin(), ord.end(), [&](int32_t a, int32_t b) { return work[a] > work[b]; });
+    std::stable_sort(ord.begin(), ord.end(), [&](int32_t a, int32_t b) {
+      if (work[a] != work[b]) return work[a] > work[b];
+      const BModel &ma = bm[bt[a].model], &mb = bm[bt[b].model];
+      return ma.n_bip != mb.n_bip ? ma.n_bip > mb.n_bip : ma.n_ev > mb.n_ev;
+    });
     std::vector<BTile> sorted(bt.size());
     for (size_t i = 0; i < ord.size(); ++i) sorted[i] = bt[ord[i]];
     bt.swap(sorted);
