@@ -117,6 +117,7 @@ struct PrepArgs {
   int32_t* flags;  // [0]: non-separable beams seen
   int32_t input_plane;  // 1: field of the beams in their own plane (no model)
   int32_t unit_amp;     // 1: every amplitude taken as 1 (the field adjoint's records)
+  BeamFast* unit;       // when given: the records of unit amplitudes too
 };
 
 __global__ void __launch_bounds__(128)
@@ -221,6 +222,7 @@ k_field_prep(const __grid_constant__ DModel M, const __grid_constant__ PrepArgs 
   // Phase polynomial (k/2) (s^T S s + L.s + c0) of the pixel position r,
   // s = r - origin, and the prefactor pref:
   cd Sxx, Syy, Sxy, Lx, Ly, c0, pref;
+  cd root = C(1.0);  // pref = amp / root
   double ox, oy;
   if (A.input_plane) {
     // the beams in their own plane (gaussian.py:402-409): s = r1 - r1m,
@@ -240,7 +242,8 @@ k_field_prep(const __grid_constant__ DModel M, const __grid_constant__ PrepArgs 
     const double r2mx = m[0][0] * x0 + m[0][1] * y0 + m[0][2] * dx0 + m[0][3] * dy0;
     const double r2my = m[1][0] * x0 + m[1][1] * y0 + m[1][2] * dx0 + m[1][3] * dy0;
     const cd det = denom.a * denom.d - denom.b * denom.c;
-    pref = cdiv(amp, csqrt_(det));
+    root = csqrt_(det);
+    pref = cdiv(amp, root);
     const cm2 ABinv = mm(Am, Binv);
     const cm2 P = mm(Q1, inv2c(mm(Bm, madd(mm(Am, Q1), Bm))));
     // quadratic (symmetric part), linear and constant terms in s = r2 - e
@@ -320,6 +323,12 @@ k_field_prep(const __grid_constant__ DModel M, const __grid_constant__ PrepArgs 
     f.rho_im = (float)(mag * sa);
   }
   A.fast[b] = f;
+  if (A.unit) {  // only the constants of the phase and of the envelope differ
+    const cd up = A.input_plane ? C(1.0) : cdiv(C(1.0), root);
+    f.p_0 = to_turns(k_0.re) + to_turns(ph_off) + to_turns(atan2(up.im, up.re));
+    f.e0 = (float)(log(hypot(up.re, up.im)) - imphi_c);
+    A.unit[b] = f;
+  }
   if (k_rc.re != 0.0 || k_rc.im != 0.0) atomicOr(A.flags, 1);
 }
 
@@ -863,7 +872,7 @@ extern "C" size_t tg_field_workspace(int64_t n_beams, int32_t h, int32_t w, int3
 namespace tg {
 static int field_prep_launch(const DModel& dm, const tg_beams* beams, const tg_pixel_map* pm,
                              void* workspace, size_t ws_bytes, int32_t* flags, void* stream,
-                             int input_plane, int unit_amp = 0) {
+                             int input_plane, int unit_amp = 0, void* unit = nullptr) {
   if (!beams || !pm || pm->h <= 0 || pm->w <= 0 || beams->n < 0) return TG_ERR_INVALID;
   if (beams->n > 0 && (!beams->x || !beams->y || !beams->dx || !beams->dy || !beams->pathlength ||
                        !beams->amplitude || !beams->waist_xy || !beams->radii))
@@ -895,6 +904,7 @@ static int field_prep_launch(const DModel& dm, const tg_beams* beams, const tg_p
   A.flags = fl;
   A.input_plane = input_plane;
   A.unit_amp = unit_amp;
+  A.unit = reinterpret_cast<BeamFast*>(unit);
   // 64-thread blocks: one thread per beam is all the parallelism there is, so
   // spread the (float64-bound) beams over every SM
   int blocks = (int)((beams->n + 63) / 64);
@@ -923,6 +933,22 @@ extern "C" int tg_field_prep(const tg_model* model, const tg_beams* beams,
   int st = build_dmodel(model, beams->z, &dm);
   if (st != TG_OK) return st;
   return field_prep_launch(dm, beams, pm, workspace, ws_bytes, flags, stream, 0);
+}
+
+extern "C" size_t tg_field_unit_bytes(int64_t n_beams) {
+  return n_beams > 0 ? (size_t)n_beams * sizeof(BeamFast) : 0;
+}
+
+extern "C" int tg_field_prep_grad(const tg_model* model, const tg_beams* beams, const tg_pixel_map* pm,
+                                  void* workspace, size_t ws_bytes, int32_t* flags, void* unit, size_t unit_bytes,
+                                  void* stream) {
+  if (!model || !beams) return TG_ERR_INVALID;
+  if (!unit || unit_bytes < tg_field_unit_bytes(beams->n)) return TG_ERR_WORKSPACE;
+  if (((uintptr_t)unit & 15) != 0) return TG_ERR_ALIGN;
+  DModel dm;
+  int st = build_dmodel(model, beams->z, &dm);
+  if (st != TG_OK) return st;
+  return field_prep_launch(dm, beams, pm, workspace, ws_bytes, flags, stream, 0, 0, unit);
 }
 
 extern "C" int tg_field_prep_input(const tg_beams* beams, const tg_pixel_map* pm, void* workspace,

@@ -1123,7 +1123,8 @@ int launch_field_gemm(const __nv_bfloat16_raw* vplanes, const __nv_bfloat16_raw*
 
 static int field_vjp_impl(const tg_model* model, const tg_beams* beams, const tg_pixel_map* pm,
                           const float* grad, const tg_field_grads* out, void* workspace, size_t ws_bytes,
-                          void* stream, int method = TG_FIELD_DIRECT, const unsigned char* want = nullptr) {
+                          void* stream, int method = TG_FIELD_DIRECT, const unsigned char* want = nullptr,
+                          const void* unit = nullptr) {
   if (method != TG_FIELD_DIRECT && method != TG_FIELD_SEPARABLE) return TG_ERR_INVALID;
   if (!beams || !pm || !grad || !out || pm->h <= 0 || pm->w <= 0 || beams->n < 0) return TG_ERR_INVALID;
   const bool input_plane = model == nullptr;
@@ -1148,12 +1149,15 @@ static int field_vjp_impl(const tg_model* model, const tg_beams* beams, const tg
   if (out->raw && cudaMemsetAsync(out->raw, 0, sizeof(double) * 4 * (size_t)nsteps, s) != cudaSuccess)
     return TG_ERR_CUDA;
   if (n == 0) return TG_OK;
-  // 1. unit-amplitude records
-  int st = field_prep_unit_amp(dm, beams, pm, ws + L.rec, field_records_bytes(n), stream, input_plane ? 1 : 0);
-  if (st != TG_OK) return st;
+  // 1. unit-amplitude records, unless the forward preparation left them
+  if (!unit) {
+    int st = field_prep_unit_amp(dm, beams, pm, ws + L.rec, field_records_bytes(n), stream, input_plane ? 1 : 0);
+    if (st != TG_OK) return st;
+    unit = ws + L.rec;
+  }
   // 2. moments
   MomArgs MA;
-  MA.beams = reinterpret_cast<const BeamFast*>(ws + L.rec);
+  MA.beams = reinterpret_cast<const BeamFast*>(unit);
   MA.g = reinterpret_cast<const float2*>(grad);
   MA.n = n;
   MA.h = pm->h;
@@ -1307,9 +1311,10 @@ extern "C" int tg_field_vjp_ex(int32_t method, const tg_model* model, const tg_b
 
 extern "C" int tg_field_vjp_steps(int32_t method, const tg_model* model, const tg_beams* beams, const tg_pixel_map* pm,
                                   const float* grad, const tg_field_grads* out, const unsigned char* want,
-                                  void* workspace, size_t ws_bytes, void* stream) {
+                                  const void* unit, void* workspace, size_t ws_bytes, void* stream) {
   if (!model) return TG_ERR_INVALID;
-  return field_vjp_impl(model, beams, pm, grad, out, workspace, ws_bytes, stream, method, want);
+  if (((uintptr_t)unit & 15) != 0) return TG_ERR_ALIGN;
+  return field_vjp_impl(model, beams, pm, grad, out, workspace, ws_bytes, stream, method, want, unit);
 }
 
 extern "C" int tg_field_vjp_input_ex(int32_t method, const tg_beams* beams, const tg_pixel_map* pm,

@@ -79,7 +79,10 @@ N.register("tg_field_vjp_ex", C.c_int, [C.c_int32, C.POINTER(N.TgModel), C.POINT
                                         C.c_void_p, C.c_size_t, C.c_void_p])
 N.register("tg_field_vjp_steps", C.c_int, [C.c_int32, C.POINTER(N.TgModel), C.POINTER(TgBeams),
                                            C.POINTER(TgPixelMap), C.c_void_p, C.POINTER(TgFieldGrads),
-                                           C.c_char_p, C.c_void_p, C.c_size_t, C.c_void_p])
+                                           C.c_char_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p])
+N.register("tg_field_unit_bytes", C.c_size_t, [C.c_int64])
+N.register("tg_field_prep_grad", C.c_int, [C.POINTER(N.TgModel), C.POINTER(TgBeams), C.POINTER(TgPixelMap),
+                                           C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p])
 N.register("tg_field_vjp_input_ex", C.c_int, [C.c_int32, C.POINTER(TgBeams), C.POINTER(TgPixelMap), C.c_void_p,
                                               C.POINTER(TgFieldGrads), C.c_void_p, C.c_size_t, C.c_void_p])
 
@@ -215,7 +218,7 @@ class FieldPlan:
     the beams in their own plane (gaussian.py:372-427)."""
 
     def __init__(self, gaussian_rays: GaussianRay, model, method: str = "auto", *, grid=None,
-                 _settle: bool = True):
+                 _settle: bool = True, _unit: bool = False):
         if not isinstance(gaussian_rays, GaussianRay):
             raise TypeError("gaussian_rays must be a GaussianRay (gaussian.py:228)")
         comps = None
@@ -236,6 +239,7 @@ class FieldPlan:
         off = (-self.ws.data_ptr()) % 256
         self.ws_ptr = self.ws.data_ptr() + off
         self.ws_bytes = self.ws.numel() - off
+        self.unit = None
         self.flags = torch.empty(1, dtype=torch.int32, device=self.dev)  # written by the preparation
         if comps is None:
             st = N.lib().tg_field_prep_input(C.byref(self.beams.struct()), C.byref(self.pm), self.ws_ptr,
@@ -243,8 +247,15 @@ class FieldPlan:
             N.check(st, "tg_field_prep_input")
         else:
             m, keep = pack_model(comps)
-            st = N.lib().tg_field_prep(C.byref(m), C.byref(self.beams.struct()), C.byref(self.pm),
-                                       self.ws_ptr, self.ws_bytes, self.flags.data_ptr(), N.stream_ptr())
+            args = (C.byref(m), C.byref(self.beams.struct()), C.byref(self.pm), self.ws_ptr, self.ws_bytes,
+                    self.flags.data_ptr())
+            if _unit and self.beams.n:
+                # the records that the adjoint starts from, in the same pass
+                self.unit = torch.empty(N.lib().tg_field_unit_bytes(self.beams.n), dtype=torch.uint8,
+                                        device=self.dev)
+                st = N.lib().tg_field_prep_grad(*args, self.unit.data_ptr(), self.unit.numel(), N.stream_ptr())
+            else:
+                st = N.lib().tg_field_prep(*args, N.stream_ptr())
             del keep
             N.check(st, "tg_field_prep")
         if method == "auto":
@@ -326,7 +337,7 @@ class FieldPlan:
         else:
             m, keep = pack_model(self.comps)
             st = N.lib().tg_field_vjp_steps(code, C.byref(m), C.byref(self.beams.struct()), C.byref(self.pm),
-                                            g.data_ptr(), C.byref(out), _steps, ws.data_ptr() + off,
+                                            g.data_ptr(), C.byref(out), _steps, N.ptr(self.unit), ws.data_ptr() + off,
                                             ws.numel() - off, N.stream_ptr())
             del keep
             N.check(st, "tg_field_vjp_steps")
@@ -375,7 +386,7 @@ def _field_autograd(gaussian_rays: GaussianRay, model, method: str, grid=None):
     params = _grad_params(_check_model(model)) if model is not None else []
     if not params and all(t is None for _, t in beam_inputs):
         return None
-    plan = FieldPlan(gaussian_rays, model, method, grid=grid, _settle=False)
+    plan = FieldPlan(gaussian_rays, model, method, grid=grid, _settle=False, _unit=True)
     spec = {"plan": plan, "beam_inputs": beam_inputs, "params": params}
     tensors = [t for _, t in beam_inputs if t is not None] + [t for (_, _, t) in params]
     spec["beam_inputs"] = [(n_, t) for n_, t in beam_inputs if t is not None]

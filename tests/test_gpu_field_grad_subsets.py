@@ -72,3 +72,24 @@ def test_field_gradients_of_subsets(cuda, name, n):
         _same(_grads(name, leaves, (k,), [])[0], full[i])
     for j, p in enumerate(steps):
         _same(_grads(name, leaves, (), [p])[0], full[len(BEAM) + j])
+
+
+@pytest.mark.parametrize("name", ["image", "column"])
+@pytest.mark.parametrize("n", [1, 64, 131])
+def test_field_gradients_from_the_forward_records(cuda, name, n):
+    """The unit-amplitude records that the differentiable forward leaves are the
+    ones that the adjoint forms by itself (FieldPlan.vjp): bit for bit, NaN
+    included, and so are the beams' gradients."""
+    import temgymcore_gb300 as t
+    from temgymcore_gb300.gaussian import FieldPlan
+    beams, params = _leaves(n, n)
+    rays = t.GaussianRay(z=0.0, waist_xy=np.full((n, 2), 3e-6), radii_of_curv=np.full((n, 2), np.inf),
+                         wavelength=1.97e-12, theta=np.linspace(0.0, 1.0, n), **beams)
+    model = _model(name, params)
+    own, left = FieldPlan(rays, model), FieldPlan(rays, model, _unit=True)
+    assert own.unit is None and left.unit is not None
+    up = torch.ones(40, 36, dtype=torch.complex64, device="cuda")
+    a, b = own.vjp(up), left.vjp(up)
+    for k in a:
+        assert torch.equal(torch.nan_to_num(torch.view_as_real(a[k]) if a[k].is_complex() else a[k]),
+                           torch.nan_to_num(torch.view_as_real(b[k]) if b[k].is_complex() else b[k])), k
