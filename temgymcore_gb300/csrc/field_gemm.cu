@@ -32,6 +32,8 @@ namespace tg {
 constexpr int kGStages = 3;
 constexpr int kTileBytes = 128 * 64;            // 128 lines x 32 bf16
 constexpr int kStageBytes = 8 * kTileBytes;     // 4 V planes + [Ur;Ui] hi and lo
+constexpr int kEpiPitch = 32 * 8 + 16;  // a row of 32 output columns; a warp's 16-byte accesses without conflicts
+static_assert(4 * 128 * kEpiPitch <= kGStages * kStageBytes, "the epilogue's tile fits the stages");
 constexpr int kGemmSmem = kGStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/;
 // kind::f16 instruction descriptor: f32 accumulate, bf16 A and B, both
 // K-major, N = 256, M = 128.
@@ -174,36 +176,45 @@ k_field_gemm(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gemm
   }
   __syncwarp();
 
-  // ---------------- epilogue: TMEM -> registers -> partial image
+  // ---------------- epilogue: TMEM -> registers -> shared memory -> partial image.
+  // A thread holds a row, so it would write 16 bytes of 32 different rows at a
+  // time; through the pipeline's free stages a warp writes 256 bytes of two rows.
+  // Measured: 384 x 24,576 x 384 (the adjoint of 8,192 beams) 85 -> 66 us, 512 x 512
+  // x 2,048 with preparation of the operands and reduction 30.8 -> 26.7, x 16,384
+  // 99.3 -> 97.8.
   const bool got = mbar_wait(done, 0, &g_tg_err, TG_EW_MMA);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const int row = mt * 128 + warp * 32 + lane;
-  float2* out = A.part + (size_t)sp * A.h * A.w + (size_t)row * A.w;
+  const bool all = __all_sync(0xffffffffu, got);  // every MMA done: no copy is in flight and no stage read
   const uint32_t lane_base = ((uint32_t)(warp * 32)) << 16;
-  for (int c = 0; c < 4; ++c) {
+  uint8_t* mine = smem + warp * (128 * kEpiPitch);  // four chunks of 32 columns, each [32 rows][kEpiPitch]
+  const int row0 = mt * 128 + warp * 32, rows = A.h - row0 < 32 ? A.h - row0 : 32;
+  const bool even = (A.w & 1) == 0;  // every row starts on 16 bytes
+  for (int c = 0; c < 4; ++c, mine += 32 * kEpiPitch) {
     uint32_t a_re[32], a_im[32], b_re[32], b_im[32];
     tmem_ld32(tmem + lane_base + 0 + c * 32, a_re);    // D0: Vr Ur
     tmem_ld32(tmem + lane_base + 128 + c * 32, a_im);  // D0: Vr Ui
     tmem_ld32(tmem + lane_base + 256 + c * 32, b_re);  // D1: Vi Ur
     tmem_ld32(tmem + lane_base + 384 + c * 32, b_im);  // D1: Vi Ui
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-    const int col0 = nt * 128 + c * 32;
-    if (got && row < A.h) {
-      if (col0 + 32 <= A.w && (A.w & 1) == 0) {
+    if (!all) continue;
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          float4 v = make_float4(__uint_as_float(a_re[j]) - __uint_as_float(b_im[j]),
-                                 __uint_as_float(a_im[j]) + __uint_as_float(b_re[j]),
-                                 __uint_as_float(a_re[j + 1]) - __uint_as_float(b_im[j + 1]),
-                                 __uint_as_float(a_im[j + 1]) + __uint_as_float(b_re[j + 1]));
-          *reinterpret_cast<float4*>(out + col0 + j) = v;
-        }
-      } else {
-        for (int j = 0; j < 32; ++j)
-          if (col0 + j < A.w)
-            out[col0 + j] = make_float2(__uint_as_float(a_re[j]) - __uint_as_float(b_im[j]),
-                                        __uint_as_float(a_im[j]) + __uint_as_float(b_re[j]));
-      }
+    for (int j = 0; j < 32; j += 2)
+      *reinterpret_cast<float4*>(mine + lane * kEpiPitch + j * 8) =
+          make_float4(__uint_as_float(a_re[j]) - __uint_as_float(b_im[j]),
+                      __uint_as_float(a_im[j]) + __uint_as_float(b_re[j]),
+                      __uint_as_float(a_re[j + 1]) - __uint_as_float(b_im[j + 1]),
+                      __uint_as_float(a_im[j + 1]) + __uint_as_float(b_re[j + 1]));
+    __syncwarp();
+    const int col0 = nt * 128 + c * 32, cols = A.w - col0 < 32 ? A.w - col0 : 32;
+    float2* out = A.part + (size_t)sp * A.h * A.w + (size_t)row0 * A.w + col0;
+    if (even) {
+      const int k = lane & 15;
+      if (2 * k < cols)
+        for (int r = lane >> 4; r < rows; r += 2)
+          reinterpret_cast<float4*>(out + (size_t)r * A.w)[k] = reinterpret_cast<const float4*>(mine + r * kEpiPitch)[k];
+    } else if (lane < cols) {
+      for (int r = 0; r < rows; ++r)
+        out[(size_t)r * A.w + lane] = reinterpret_cast<const float2*>(mine + r * kEpiPitch)[lane];
     }
   }
   // drain: a producer that issued loads must see them land before the CTA exits
