@@ -63,18 +63,6 @@ class Component(HasParamsMixin):
         for i, v in enumerate(self._params()):
             comp.p[i] = v
 
-    def _packed(self) -> bytes:
-        """The packed TgComponent: kept on the instance while its fields are
-        plain numbers (frozen), formed anew where a field may change."""
-        b = self.__dict__.get("_packed_cache")
-        if b is None:
-            comp = N.TgComponent()
-            self._pack(comp)
-            b = bytes(comp)
-            if _frozen(self):
-                object.__setattr__(self, "_packed_cache", b)
-        return b
-
     def new_with(self, **kw):
         """tree_utils.py:168-172."""
         return dataclasses.replace(self, **kw)
