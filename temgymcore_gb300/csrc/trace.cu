@@ -176,7 +176,7 @@ __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, con
       // so base + plv is rounded with float32 / integer operations.  The two
       // cases are separate loops: as selects on one loop's base the compiler
       // ran the float64 adds for every ray (a quarter of the float64 pipe at
-      // 8 M rays through eight components, 88 -> 77 us without them)
+      // 8 M rays through eight components, 86.7 -> 81.3 us without them)
       double o[R];
       if (A.pl || A.z) {
 #pragma unroll
@@ -1068,17 +1068,23 @@ __device__ __forceinline__ void lean_reverse(const Op& op, Ray4& r, Ray4& a, flo
 // evict-first loads and stores 0.157 ms (three blocks 0.189 ms).
 constexpr int kLeanRays = 8;    // rays per thread
 constexpr int kLeanBlocks = 2;  // resident blocks per SM (register bound)
+// Steps up to which a chain with every gradient given takes the short form, a
+// dispatch per ray and step: slower code, but two components are bound by memory,
+// where the quicker form mixes the blocks' reads and writes more.  Lens + Detector,
+// short / quick: 2 M rays 24.9 / 25.8 us, 8 M 71.1 / 73.1, 16.8 M 127.8 / 135.4
+// (130 with a barrier a turn); three components, 16.8 M: 141 / 131.
+constexpr int kLeanShort = 4;
 
-// One component at a time, its kind decided once for all R rays of a thread
-// (both ways: its free-space step and its own).  The sums run in the general
-// kernel's order (a thread's rays, the warp, the block's turns in float32; warps
-// and blocks in float64), so they equal its sums bit for bit.  16.8 M rays,
-// Lens + Detector: 130 us, 0.92 of measured HBM.  2.1 M rays through five
-// components with every gradient given 34.8 us (a dispatch per ray and step
-// 35.9), with those of x and y alone 31.7 (the general kernel, which gradients
-// of zeros used to take, 49.3); one block a tile, handed out by the hardware,
-// 44 and 170 us (a block's start is not hidden by two blocks an SM).
-template <int R>
+// One component at a time, its kind decided once for all R rays of a thread (both
+// ways: its free-space step and its own; kShort: step by step).  The sums run in
+// the general kernel's order (a thread's rays, the warp, the block's turns in
+// float32; warps and blocks in float64), so they equal its sums bit for bit.
+// 16.8 M rays, Lens + Detector (kShort): 127 us, 0.93 of measured HBM.  2.1 M rays
+// through five components with every gradient given 33.8-34.8 us (a dispatch per
+// ray and step 35.9), with those of x and y alone 31.7 (the general kernel, which
+// gradients of zeros used to take, 49.3); one block a tile, handed out by the
+// hardware, 44 and 170 us (a block's start is not hidden by two blocks an SM).
+template <int R, bool kShort>
 __global__ void __launch_bounds__(kVjpThreads, kLeanBlocks)
 k_trace_vjp_lean(const __grid_constant__ Program P, const __grid_constant__ VjpArgs A) {
   extern __shared__ float wacc[];  // [warps][4 n_steps] step sums
@@ -1099,9 +1105,6 @@ k_trace_vjp_lean(const __grid_constant__ Program P, const __grid_constant__ VjpA
   for (int64_t blk = (int64_t)blockIdx.x * blockDim.x * R; blk < n; blk += stride) {
     const int64_t i0 = blk + (int64_t)threadIdx.x * R;
     const bool vec = i0 + R - 1 < n;
-    // short chains: the block's loads and stores in phases of their own (16.8 M
-    // rays, Lens + Detector: 135 -> 130 us)
-    if (P.n_steps <= 4) __syncthreads();
     Ray4 r[R], ad[R];
     {
       float x[R], y[R], dx[R], dy[R], gx[R], gy[R], gdx[R], gdy[R];
@@ -1109,10 +1112,14 @@ k_trace_vjp_lean(const __grid_constant__ Program P, const __grid_constant__ VjpA
       load4<R, true>(A.y, i0, n, y, vec);
       load4<R, true>(A.dx, i0, n, dx, vec);
       load4<R, true>(A.dy, i0, n, dy, vec);
-      load_or_zero<R, true>(A.gx, i0, n, gx, vec);
-      load_or_zero<R, true>(A.gy, i0, n, gy, vec);
-      load_or_zero<R, true>(A.gdx, i0, n, gdx, vec);
-      load_or_zero<R, true>(A.gdy, i0, n, gdy, vec);
+      if constexpr (kShort) load4<R, true>(A.gx, i0, n, gx, vec);
+      else load_or_zero<R, true>(A.gx, i0, n, gx, vec);
+      if constexpr (kShort) load4<R, true>(A.gy, i0, n, gy, vec);
+      else load_or_zero<R, true>(A.gy, i0, n, gy, vec);
+      if constexpr (kShort) load4<R, true>(A.gdx, i0, n, gdx, vec);
+      else load_or_zero<R, true>(A.gdx, i0, n, gdx, vec);
+      if constexpr (kShort) load4<R, true>(A.gdy, i0, n, gdy, vec);
+      else load_or_zero<R, true>(A.gdy, i0, n, gdy, vec);
 #pragma unroll
       for (int k = 0; k < R; ++k) {
         r[k] = Ray4{x[k], y[k], dx[k], dy[k]};
@@ -1120,44 +1127,66 @@ k_trace_vjp_lean(const __grid_constant__ Program P, const __grid_constant__ VjpA
         ad[k] = Ray4{gx[k], gy[k], gdx[k], gdy[k]};
       }
     }
-#pragma unroll 1
-    for (int s = 0; s < P.n_steps; s += 2) {
-      auto fwd = [&](const Op& c, auto kind) {
-        Op o = c;
-        o.kind = decltype(kind)::value;
+    if constexpr (kShort) {
+      for (int s = 0; s < P.n_steps; ++s) {
+        const Op op = P.op[s];
 #pragma unroll
-        for (int k = 0; k < R; ++k) lean_forward(o, r[k]);
-      };
-      if (P.op[s].kind == OP_FREE) fwd(P.op[s], OpConst<OP_FREE>());
-      const Op& c = P.op[s + 1];
-      if (c.kind == OP_LENS) fwd(c, OpConst<OP_LENS>());
-      else if (c.kind == OP_SHIFT) fwd(c, OpConst<OP_SHIFT>());
-      else if (c.kind == OP_DEFLECT) fwd(c, OpConst<OP_DEFLECT>());
-      else if (c.kind == OP_ROTATE) fwd(c, OpConst<OP_ROTATE>());
-    }
-#pragma unroll 1
-    for (int s = P.n_steps - 2; s >= 0; s -= 2) {
-      auto rev = [&](int t, const Op& c, auto kind) {
-        constexpr int K = decltype(kind)::value, NS = K == OP_SHIFT ? 4 : (K == OP_DEFLECT ? 2 : 1);
-        Op o = c;
-        o.kind = K;
-        float cs[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int k = 0; k < R; ++k) lean_forward(op, r[k]);
+      }
+      for (int s = P.n_steps - 1; s >= 0; --s) {
+        const Op op = P.op[s];
+        float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int k = 0; k < R; ++k) {
           float ck[4] = {0.f, 0.f, 0.f, 0.f};
-          lean_reverse(o, r[k], ad[k], ck);
-#pragma unroll
-          for (int j = 0; j < NS; ++j) cs[j] += ck[j];
+          lean_reverse(op, r[k], ad[k], ck);
+          c[0] += ck[0]; c[1] += ck[1]; c[2] += ck[2]; c[3] += ck[3];
         }
+        if (sums) {
+          const int ns = op_nsums(op.kind);
+          for (int j = 0; j < ns; ++j) add_sum(s, j, c[j]);
+        }
+      }
+    } else {
+#pragma unroll 1
+      for (int s = 0; s < P.n_steps; s += 2) {
+        auto fwd = [&](const Op& c, auto kind) {
+          Op o = c;
+          o.kind = decltype(kind)::value;
 #pragma unroll
-        for (int j = 0; j < NS; ++j) add_sum(t, j, cs[j]);
-      };
-      const Op& c = P.op[s + 1];
-      if (c.kind == OP_LENS) rev(s + 1, c, OpConst<OP_LENS>());
-      else if (c.kind == OP_SHIFT) rev(s + 1, c, OpConst<OP_SHIFT>());
-      else if (c.kind == OP_DEFLECT) rev(s + 1, c, OpConst<OP_DEFLECT>());
-      else if (c.kind == OP_ROTATE) rev(s + 1, c, OpConst<OP_ROTATE>());
-      if (P.op[s].kind == OP_FREE) rev(s, P.op[s], OpConst<OP_FREE>());
+          for (int k = 0; k < R; ++k) lean_forward(o, r[k]);
+        };
+        if (P.op[s].kind == OP_FREE) fwd(P.op[s], OpConst<OP_FREE>());
+        const Op& c = P.op[s + 1];
+        if (c.kind == OP_LENS) fwd(c, OpConst<OP_LENS>());
+        else if (c.kind == OP_SHIFT) fwd(c, OpConst<OP_SHIFT>());
+        else if (c.kind == OP_DEFLECT) fwd(c, OpConst<OP_DEFLECT>());
+        else if (c.kind == OP_ROTATE) fwd(c, OpConst<OP_ROTATE>());
+      }
+#pragma unroll 1
+      for (int s = P.n_steps - 2; s >= 0; s -= 2) {
+        auto rev = [&](int t, const Op& c, auto kind) {
+          constexpr int K = decltype(kind)::value, NS = K == OP_SHIFT ? 4 : (K == OP_DEFLECT ? 2 : 1);
+          Op o = c;
+          o.kind = K;
+          float cs[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int k = 0; k < R; ++k) {
+            float ck[4] = {0.f, 0.f, 0.f, 0.f};
+            lean_reverse(o, r[k], ad[k], ck);
+#pragma unroll
+            for (int j = 0; j < NS; ++j) cs[j] += ck[j];
+          }
+#pragma unroll
+          for (int j = 0; j < NS; ++j) add_sum(t, j, cs[j]);
+        };
+        const Op& c = P.op[s + 1];
+        if (c.kind == OP_LENS) rev(s + 1, c, OpConst<OP_LENS>());
+        else if (c.kind == OP_SHIFT) rev(s + 1, c, OpConst<OP_SHIFT>());
+        else if (c.kind == OP_DEFLECT) rev(s + 1, c, OpConst<OP_DEFLECT>());
+        else if (c.kind == OP_ROTATE) rev(s + 1, c, OpConst<OP_ROTATE>());
+        if (P.op[s].kind == OP_FREE) rev(s, P.op[s], OpConst<OP_FREE>());
+      }
     }
     float o[R];
 #pragma unroll
@@ -1281,7 +1310,11 @@ static int trace_vjp_impl(const tg_model* model, const tg_rays* in, const tg_ray
   const bool opt = !A.gx || !A.gy || !A.gdx || !A.gdy;
   if (lean) {
     const size_t smem = sizeof(float) * (kVjpThreads / 32) * 4 * (size_t)P.n_steps;  // at most 15 KB
-    k_trace_vjp_lean<kLeanRays><<<grid, kVjpThreads, A.partial ? smem : 0, s>>>(P, A);
+    const size_t dyn = A.partial ? smem : 0;
+    if (P.n_steps <= kLeanShort && !opt)
+      k_trace_vjp_lean<kLeanRays, true><<<grid, kVjpThreads, dyn, s>>>(P, A);
+    else
+      k_trace_vjp_lean<kLeanRays, false><<<grid, kVjpThreads, dyn, s>>>(P, A);
   } else if (P.n_aber > 0) {
     if (vec) vjp_launch<4, true>(P, A, grid, opt, s);
     else vjp_launch<1, true>(P, A, grid, opt, s);
