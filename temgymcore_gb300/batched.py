@@ -97,7 +97,7 @@ class BatchedTrace:
         self.offsets = np.concatenate([[0], np.cumsum(self.n_rays)])
         self.total = int(self.offsets[-1])
         self.step_offsets = np.concatenate([[0], np.cumsum([2 * len(m) for m in self.models])])
-        self._packed = [pack_model(m, keep=False) for m in self.models]
+        self._packed = [pack_model(m) for m in self.models]
         self._build(tile_rays)
         self.block, self.rpt = 256, 2
         self.graph = None

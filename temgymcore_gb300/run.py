@@ -15,7 +15,7 @@ import numpy as np
 import torch
 
 from . import _native as N
-from .components import Component, DescanError, Descanner, Grid, ThickLens, Source, _f, _frozen
+from .components import Component, DescanError, Descanner, Grid, ThickLens, Source, _f
 from .propagator import FreeSpaceDirCosine, FreeSpaceParaxial, Propagator
 from .ray import Ray, as_f32, as_f64_or_scalar
 
@@ -43,38 +43,19 @@ def _prop_code(propagator) -> int:
     raise NotImplementedError(f"{type(propagator).__name__} is not a GPU propagator")
 
 
-def pack_components(comps, keep=True):
-    """The component table of a checked model (ctypes array, at least one entry).
-    A component whose fields are plain numbers (frozen) keeps its packed bytes
-    from the second time on; others are packed anew each time.  ``keep`` False:
-    neither used nor kept (a sweep packs its many components once)."""
-    arr = N.TgComponent * max(1, len(comps))
-    if not keep:
-        table = arr()
-        for i, c in enumerate(comps):
-            c._pack(table[i])
-        return table
-    kept = [c.__dict__.get("_packed_cache") for c in comps]
-    if kept and all(kept):
-        return arr.from_buffer_copy(b"".join(kept))
-    table = arr()
-    for i, (c, b) in enumerate(zip(comps, kept)):
-        if b:
-            C.memmove(C.byref(table[i]), b, len(b))
-            continue
+def pack_components(comps):
+    """The component table of a checked model (ctypes array, at least one entry)."""
+    table = (N.TgComponent * max(1, len(comps)))()
+    for i, c in enumerate(comps):
         c._pack(table[i])
-        if b is None:  # first time
-            c.__dict__["_packed_cache"] = b""
-        elif b == b"":  # second time (0: a field may change, never kept)
-            c.__dict__["_packed_cache"] = bytes(table[i]) if _frozen(c) else 0
     return table
 
 
-def pack_model(model, propagator=None, keep=True):
+def pack_model(model, propagator=None):
     """(TgModel, keep-alive array) for a sequence of components; ``propagator``
     selects the free-space model between them (default paraxial)."""
     comps = _check_model(model)
-    arr = pack_components(comps, keep)
+    arr = pack_components(comps)
     m = N.TgModel()
     m.n_components = len(comps)
     m.propagator = _prop_code(propagator)

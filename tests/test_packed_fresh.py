@@ -1,0 +1,51 @@
+"""Components are read at every call: nothing that follows from their fields is kept
+on them, whatever way a field is set or computed (CPU only)."""
+import copy
+import dataclasses
+
+import pytest
+
+import temgymcore_gb300 as t
+from temgymcore_gb300.run import pack_model
+from temgymcore_gb300.scan import pack_scan_model
+
+
+def _focal(lens, pack):
+    _, arr = pack([lens])
+    return arr[0].p[0]
+
+
+class _Computed(t.Lens):
+    """A plain subclass (it inherits the frozen dataclass) that computes its setting."""
+    setting = 0.2
+
+    def _params(self):
+        return [type(self).setting]
+
+
+@pytest.mark.parametrize("pack", [pack_model, pack_scan_model])
+def test_a_setting_that_moves_is_packed_at_every_call(pack):
+    lens = _Computed(z=0.5, focal_length=1.0)
+    for v in (0.2, 0.3, 0.4, 0.5):
+        _Computed.setting = v
+        assert _focal(lens, pack) == v
+
+
+@pytest.mark.parametrize("pack", [pack_model, pack_scan_model])
+def test_a_frozen_field_that_is_set_all_the_same_is_packed(pack):
+    lens = t.Lens(z=0.5, focal_length=0.2)
+    for v in (0.2, 0.2, 0.3, 0.4):
+        object.__setattr__(lens, "focal_length", v)
+        assert _focal(lens, pack) == v
+    other = copy.copy(lens)
+    object.__setattr__(other, "focal_length", 0.6)
+    assert _focal(other, pack) == 0.6 and _focal(lens, pack) == 0.4
+
+
+def test_packing_leaves_nothing_on_a_component():
+    det = t.Detector(z=1.0, pixel_size=(1e-5, 2e-5), shape=(8, 9))
+    lens = t.Lens(z=0.5, focal_length=0.2)
+    for _ in range(3):
+        pack_model([lens, det])
+    names = {f.name for c in (lens, det) for f in dataclasses.fields(c)}
+    assert set(lens.__dict__) <= names and set(det.__dict__) <= names
