@@ -27,19 +27,6 @@ def _f(v) -> float:
     return float(v)
 
 
-def _plain(v) -> bool:
-    """True for values that cannot change in place: numbers, and tuples of them."""
-    return isinstance(v, (int, float, np.generic)) or v is None or (isinstance(v, tuple) and all(map(_plain, v)))
-
-
-def _frozen(obj) -> bool:
-    """True for an instance of a frozen dataclass whose fields cannot change
-    in place: what follows from them alone may be kept on the instance."""
-    params = getattr(obj, "__dataclass_params__", None)
-    return (params is not None and params.frozen
-            and all(_plain(getattr(obj, f)) for f in obj.__dataclass_fields__))
-
-
 class Component(HasParamsMixin):
     """Base component: ``__call__(ray) -> Ray`` (components.py:12-24)."""
 
@@ -205,15 +192,9 @@ class Grid:
         return g
 
     def _pixel_map(self) -> tuple:
-        """The six numbers of the pixels -> metres map (y row, then x row),
-        kept on the instance while its fields are plain numbers."""
-        t = self.__dict__.get("_pixel_map_cache")
-        if t is None:
-            m = self.pixels_to_metres_mat
-            t = tuple(float(v) for v in (m[0, 0], m[0, 1], m[0, 2], m[1, 0], m[1, 1], m[1, 2]))
-            if _frozen(self):
-                object.__setattr__(self, "_pixel_map_cache", t)
-        return t
+        """The six numbers of the pixels -> metres map (y row, then x row)."""
+        m = self.pixels_to_metres_mat
+        return tuple(float(v) for v in (m[0, 0], m[0, 1], m[0, 2], m[1, 0], m[1, 1], m[1, 2]))
 
     @property
     def coords_px(self):

@@ -1,11 +1,12 @@
-"""Components are read at every call: nothing that follows from their fields is kept
-on them, whatever way a field is set or computed (CPU only)."""
+"""Components and grids are read at every call: nothing that follows from their fields
+is kept on them, whatever way a field is set or computed (CPU only)."""
 import copy
 import dataclasses
 
 import pytest
 
 import temgymcore_gb300 as t
+from temgymcore_gb300.gaussian import pixel_map
 from temgymcore_gb300.run import pack_model
 from temgymcore_gb300.scan import pack_scan_model
 
@@ -49,3 +50,12 @@ def test_packing_leaves_nothing_on_a_component():
         pack_model([lens, det])
     names = {f.name for c in (lens, det) for f in dataclasses.fields(c)}
     assert set(lens.__dict__) <= names and set(det.__dict__) <= names
+
+
+def test_the_pixel_map_follows_the_grid():
+    det = t.Detector(z=1.0, pixel_size=(1e-5, 2e-5), shape=(8, 9))
+    pixel_map(det)
+    for grid in (det, copy.copy(det)):
+        object.__setattr__(grid, "pixel_size", (3e-5, 4e-5))
+        assert list(pixel_map(grid).t) == list(pixel_map(dataclasses.replace(grid)).t)
+    assert set(det.__dict__) <= {f.name for f in dataclasses.fields(det)}
