@@ -120,9 +120,6 @@ class GaussianRay(Ray):
     def size(self) -> int:
         """Number of beams: per-beam fields have length n; waist_xy and
         radii_of_curv are (n, 2)."""
-        cached = self.__dict__.get("_size_cache")  # fields are frozen: computed once
-        if cached is not None:
-            return cached
         sizes = set()
         for f in dataclasses.fields(self):
             v = getattr(self, f.name)
@@ -134,9 +131,7 @@ class GaussianRay(Ray):
                 sizes.add(_size(v))
         sizes.discard(1) if len(sizes) > 1 else None
         assert len(sizes) <= 1, "beam fields have mismatched sizes"
-        n = sizes.pop() if sizes else 1
-        object.__setattr__(self, "_size_cache", n)
-        return n
+        return sizes.pop() if sizes else 1
 
     def derive(self, **updates):
         return dataclasses.replace(self, **{k: (v(self) if callable(v) else v)

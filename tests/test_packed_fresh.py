@@ -1,9 +1,11 @@
-"""Components and grids are read at every call: nothing that follows from their fields
-is kept on them, whatever way a field is set or computed (CPU only)."""
+"""Components, grids and beams are read at every call: nothing that follows from
+their fields is kept on them, whatever way a field is set or computed (CPU only)."""
 import copy
 import dataclasses
 
+import numpy as np
 import pytest
+import torch
 
 import temgymcore_gb300 as t
 from temgymcore_gb300.gaussian import pixel_map
@@ -59,3 +61,16 @@ def test_the_pixel_map_follows_the_grid():
         object.__setattr__(grid, "pixel_size", (3e-5, 4e-5))
         assert list(pixel_map(grid).t) == list(pixel_map(dataclasses.replace(grid)).t)
     assert set(det.__dict__) <= {f.name for f in dataclasses.fields(det)}
+
+
+def test_the_number_of_beams_follows_the_fields():
+    def beams(n):
+        return {k: torch.zeros(n, dtype=torch.float64) for k in ("x", "y", "dx", "dy", "pathlength")}
+
+    b = t.GaussianRay(z=0.0, amplitude=1.0, waist_xy=np.ones((1, 2)), radii_of_curv=np.ones((1, 2)),
+                      wavelength=1e-9, theta=0.0, **beams(5))
+    assert b.size == 5
+    for r in (copy.copy(b), b):
+        for k, v in beams(7).items():
+            object.__setattr__(r, k, v)
+        assert r.size == 7
