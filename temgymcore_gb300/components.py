@@ -327,9 +327,13 @@ class Descanner(Component):
     _kind = N.DESCANNER
 
     def _params(self) -> list:
-        e = [_f(v) for v in self.descan_error]  # p[]: scan, then as_matrix4 row by row, then the offsets
-        return [_f(self.scan_pos_x), _f(self.scan_pos_y), _f(self.scan_tilt_x), _f(self.scan_tilt_y),
-                e[0], e[1], e[12], e[13], e[2], e[3], e[14], e[15], e[4], e[5], e[16], e[17],
+        # p[]: scan, then as_matrix4 row by row, then the offsets
+        scan = [_f(self.scan_pos_x), _f(self.scan_pos_y), _f(self.scan_tilt_x), _f(self.scan_tilt_y)]
+        d = self.descan_error
+        if type(d) is not DescanError:  # its own matrix and offsets
+            return scan + list(np.asarray(d.as_matrix4()).reshape(-1)) + list(d.offsets())
+        e = [_f(v) for v in d]
+        return [*scan, e[0], e[1], e[12], e[13], e[2], e[3], e[14], e[15], e[4], e[5], e[16], e[17],
                 e[6], e[7], e[18], e[19], *e[8:12]]
 
 

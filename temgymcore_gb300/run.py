@@ -161,15 +161,13 @@ def _grad_params(comps) -> list:
     """(component index, path, tensor) for every parameter tensor needing grad."""
     out = []
     for i, c in enumerate(comps):
-        if not any(isinstance(v, (torch.Tensor, DescanError)) for v in c.__dict__.values()):
-            continue
         names = [f for f in getattr(c, "__dataclass_fields__", {})]
         for name in names:
             v = getattr(c, name)
             if isinstance(v, torch.Tensor) and v.requires_grad:
                 out.append((i, name, v))
             if name == "descan_error":
-                if not any(isinstance(e, torch.Tensor) for e in v):
+                if type(v) is DescanError and not any(isinstance(e, torch.Tensor) for e in v):
                     continue
                 for dn in _DESCAN_FIELDS:
                     dv = getattr(v, dn)
