@@ -76,11 +76,11 @@ __device__ __forceinline__ DF df_norm(DF a) {
 // |lo| <= ulp32(hi) / 2, so in units of hi's float64 ulp, 2^(e - 52), lo is a
 // number below 2^28: lo times the power of two, cut to an integer, is added to
 // hi's float64 bits.  A lo that reduces a power of two leaves hi's binade, where
-// the grid is twice as fine and lo counts double.  |hi| < 2^-75 (no such power of
+// the grid is twice as fine and lo counts double.  |hi| < 2^-74 (no such power of
 // two in float32; zero) and non-finite parts take the general rounding.
 __device__ __forceinline__ double df_to_double(float h, float l) {
   const uint32_t hb = __float_as_uint(h), lb = __float_as_uint(l);
-  if ((hb & 0x7fffffffu) - (52u << 23) >= (203u << 23)) {
+  if ((hb & 0x7fffffffu) - (53u << 23) >= (202u << 23)) {
     if ((hb << 1) == 0u) return __longlong_as_double((long long)((uint64_t)(hb + lb) << 32));  // lo is 0 too
     return add_f64_f32(f32_to_f64(h), l);
   }

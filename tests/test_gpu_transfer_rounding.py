@@ -1,0 +1,34 @@
+"""GPU: the last step of the double-float transfer, a pair of float32 to one float64.
+
+The products and sums here are exact in a float32 pair, so the expected value is
+exact too and no tolerance is needed."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _out(rays, mats):
+    import temgymcore_gb300 as t
+    return t.transfer_rays(rays, mats).cpu().numpy()
+
+
+def _scaled(c, full):
+    """Every component times c (the last row too with full)."""
+    m = np.diag([c, c, c, c, 1.0])
+    if full:
+        m[4] = [c, 0.0, 0.0, 0.0, 0.0]
+    return m[None]
+
+
+@pytest.mark.parametrize("full", [False, True])
+@pytest.mark.parametrize("e", [-78, -77, -76, -75, -74, -73, -1, 0, 1])
+def test_a_power_of_two_with_a_tail_of_the_other_sign(cuda, e, full):
+    """hi = 2^e, lo = -2^(e - 30): the scale of the tail is at the edge of float32 at e = -75."""
+    entry, comp = 2.0 ** (e // 2) * (1.0 - 2.0 ** -30), 2.0 ** (e - e // 2)
+    rays = np.ones((5, 5))
+    rays[:, :4] = comp * np.array([1.0, -1.0, 1.0, -1.0])
+    rays[4, :4] = 0.0
+    out = _out(rays, _scaled(entry, full))[:, 0]
+    assert np.array_equal(out[:, :4], rays[:, :4] * entry)
+    assert np.array_equal(out[:, 4], rays[:, 0] * entry if full else rays[:, 4])
