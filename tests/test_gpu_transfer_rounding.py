@@ -32,3 +32,25 @@ def test_a_power_of_two_with_a_tail_of_the_other_sign(cuda, e, full):
     out = _out(rays, _scaled(entry, full))[:, 0]
     assert np.array_equal(out[:, :4], rays[:, :4] * entry)
     assert np.array_equal(out[:, 4], rays[:, 0] * entry if full else rays[:, 4])
+
+
+@pytest.mark.parametrize("full", [False, True])
+def test_a_sum_of_two_floats_is_rounded_to_nearest(cuda, full):
+    """x' = x + dx of two float32 values is exact as a pair: the float64 sum of
+    them is the result, for a tail of any size and sign and for powers of two."""
+    r = np.random.default_rng(0)
+    n = 20_000
+    big = (r.uniform(1.0, 2.0, (2, n)) * 2.0 ** r.integers(0, 11, (2, n))).astype(np.float32)
+    big[:, ::4] = 2.0 ** r.integers(0, 11, (2, n))[:, ::4]
+    small = (r.uniform(1.0, 2.0, (2, n)) * 2.0 ** r.integers(-38, -16, (2, n))).astype(np.float32)
+    rays = np.ones((n, 5))
+    rays[:, :2] = (big * r.choice([-1, 1], (2, n))).T
+    rays[:, 2:4] = (small * r.choice([-1, 1], (2, n))).T
+    m = np.eye(5)
+    m[0, 2] = m[1, 3] = 1.0
+    if full:
+        m[4] = [1.0, 0.0, 1.0, 0.0, 0.0]
+    out = _out(rays, m[None])[:, 0]
+    assert np.array_equal(out[:, :2], rays[:, :2] + rays[:, 2:4])
+    assert np.array_equal(out[:, 2:4], rays[:, 2:4])
+    assert np.array_equal(out[:, 4], rays[:, 0] + rays[:, 2] if full else rays[:, 4])
