@@ -192,6 +192,19 @@ class BeamSet:
         """Rotation per beam."""
         return torch.zeros_like(self.x) if self._theta is None else self._theta
 
+    def own(self) -> "BeamSet":
+        """The same values in arrays that nothing else holds (an array already in
+        the kernel layout is the caller's own until then)."""
+        parts = [t for t in (self.x, self.y, self.dx, self.dy, self.pl, self.waist, self.radii, self._wl, self._theta)
+                 if t is not None]
+        flat = [t.reshape(-1) for t in parts]
+        own = iter(torch.cat(flat).split([t.numel() for t in flat]))
+        self.x, self.y, self.dx, self.dy, self.pl = (next(own) for _ in range(5))
+        self.waist, self.radii = next(own).view(self.n, 2), next(own).view(self.n, 2)
+        self._wl, self._theta = (None if t is None else next(own) for t in (self._wl, self._theta))
+        self.amp = self.amp.clone()
+        return self
+
     def struct(self) -> TgBeams:
         b = TgBeams()
         b.n = self.n
@@ -232,6 +245,7 @@ class FieldPlan:
                 raise ValueError("the last model element must be a Detector grid (gaussian.py:231-232)")
         self.dev = _device()
         self.beams = BeamSet(gaussian_rays, self.dev)
+        self._packed = None
         self.pm = pixel_map(grid)
         self.shape = (int(grid.shape[0]), int(grid.shape[1]))
         sizes = [N.lib().tg_field_workspace(self.beams.n, self.pm.h, self.pm.w, m) for m in (0, 1, 2)]
@@ -246,17 +260,20 @@ class FieldPlan:
                                              self.ws_bytes, self.flags.data_ptr(), N.stream_ptr())
             N.check(st, "tg_field_prep_input")
         else:
-            m, keep = pack_model(comps)
-            args = (C.byref(m), C.byref(self.beams.struct()), C.byref(self.pm), self.ws_ptr, self.ws_bytes,
-                    self.flags.data_ptr())
+            packed = pack_model(comps)
             if _unit and self.beams.n:
-                # the records that the adjoint starts from, in the same pass
+                # The records that the adjoint starts from, in the same pass.  Its chain
+                # rule has to see the same beams and model: both are kept as they are now.
+                self._packed = packed
+                self.beams.own()
+            args = (C.byref(packed[0]), C.byref(self.beams.struct()), C.byref(self.pm), self.ws_ptr, self.ws_bytes,
+                    self.flags.data_ptr())
+            if self._packed is not None:
                 self.unit = torch.empty(N.lib().tg_field_unit_bytes(self.beams.n), dtype=torch.uint8,
                                         device=self.dev)
                 st = N.lib().tg_field_prep_grad(*args, self.unit.data_ptr(), self.unit.numel(), N.stream_ptr())
             else:
                 st = N.lib().tg_field_prep(*args, N.stream_ptr())
-            del keep
             N.check(st, "tg_field_prep")
         if method == "auto":
             self._method = None
@@ -335,11 +352,10 @@ class FieldPlan:
                                                ws.numel() - off, N.stream_ptr())
             N.check(st, "tg_field_vjp_input_ex")
         else:
-            m, keep = pack_model(self.comps)
-            st = N.lib().tg_field_vjp_steps(code, C.byref(m), C.byref(self.beams.struct()), C.byref(self.pm),
+            packed = self._packed or pack_model(self.comps)
+            st = N.lib().tg_field_vjp_steps(code, C.byref(packed[0]), C.byref(self.beams.struct()), C.byref(self.pm),
                                             g.data_ptr(), C.byref(out), _steps, N.ptr(self.unit), ws.data_ptr() + off,
                                             ws.numel() - off, N.stream_ptr())
-            del keep
             N.check(st, "tg_field_vjp_steps")
         return res
 
@@ -369,7 +385,7 @@ class _FieldFn(torch.autograd.Function):
                 g = g.sum()
             out.append(g.to(t.dtype).reshape(t.shape))
         if spec["params"]:
-            out += param_gradients(plan.comps, spec["params"], r["raw"])
+            out += param_gradients(plan.comps, spec["params"], r["raw"], plan._packed and plan._packed[1])
         return (None, *out)
 
 

@@ -176,9 +176,11 @@ def _grad_params(comps) -> list:
     return out
 
 
-def param_gradient(comps, i, path, raw):
+def param_gradient(comps, i, path, raw, table=None):
     """dL/d(parameter) from the adjoint's per-step sums raw[(2*n_components), 4]
-    (a float64 tensor, or a NumPy array of the sums read back to the host)."""
+    (a float64 tensor, or a NumPy array of the sums read back to the host).
+    ``table``: the component table that the sums belong to, where the
+    components may have changed since (else their present values are taken)."""
     c = comps[i]
     nc = len(comps)
     if path in ("z", "z_po"):
@@ -199,7 +201,7 @@ def param_gradient(comps, i, path, raw):
         g4 = comp[0:4]
         sp = ("scan_pos_x", "scan_pos_y", "scan_tilt_x", "scan_tilt_y")
         if path in sp:
-            m = c.descan_error.as_matrix4()
+            m = c.descan_error.as_matrix4() if table is None else np.array(table[i].p[4:20]).reshape(4, 4)
             if isinstance(raw, torch.Tensor):
                 m = torch.as_tensor(m, dtype=torch.float64, device=raw.device)
             j = sp.index(path)
@@ -208,14 +210,14 @@ def param_gradient(comps, i, path, raw):
         pos = _DESCAN_POS[dn]
         if pos[0] == "off":
             return g4[pos[1]]
-        return g4[pos[0]] * _f(getattr(c, sp[pos[1]]))
+        return g4[pos[0]] * (_f(getattr(c, sp[pos[1]])) if table is None else table[i].p[pos[1]])
     sp = {"scan_pos_x": 0, "scan_pos_y": 1, "scan_tilt_x": 2, "scan_tilt_y": 3}
     if path in sp:
         return comp[sp[path]]
     raise NotImplementedError(f"no gradient rule for {type(c).__name__}.{path}")
 
 
-def param_gradients(comps, plist, raw) -> list:
+def param_gradients(comps, plist, raw, table=None) -> list:
     """The gradients of the parameter tensors of ``plist`` (_grad_params) from
     the adjoint's per-step sums, each with its tensor's type and shape.
     Host tensors take theirs from ONE readback of the sums (a copy and a wait
@@ -224,9 +226,9 @@ def param_gradients(comps, plist, raw) -> list:
     out = []
     for i, path, t in plist:
         if t.is_cuda:
-            out.append(param_gradient(comps, i, path, raw).to(t.dtype).reshape(t.shape))
+            out.append(param_gradient(comps, i, path, raw, table).to(t.dtype).reshape(t.shape))
         else:
-            g = torch.tensor(float(param_gradient(comps, i, path, host)), dtype=t.dtype)
+            g = torch.tensor(float(param_gradient(comps, i, path, host, table)), dtype=t.dtype)
             out.append(g if t.dim() == 0 else g.reshape(t.shape))
     return out
 
