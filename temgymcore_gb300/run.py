@@ -97,6 +97,12 @@ class _Soa:
         return _rays_struct(self.n, self.x, self.y, self.dx, self.dy, self.z_t, self.z_s,
                             self.pl_t, self.pl_s, self.amp)
 
+    def versions(self) -> list:
+        """Counts of the in-place changes of the arrays that the adjoint reads
+        (they may be the caller's own)."""
+        return [None if t is None or t.is_inference() else t._version
+                for t in (self.x, self.y, self.dx, self.dy, self.z_t)]
+
 
 def _ray_scalar_input(ray: Ray) -> bool:
     return all(not isinstance(getattr(ray, f), (torch.Tensor, np.ndarray)) or
@@ -259,6 +265,7 @@ class _TraceFn(torch.autograd.Function):
     def forward(ctx, spec, x, y, dx, dy, pl, zin, *params):
         comps, soa = spec["comps"], spec["soa"]
         spec["packed"] = pack_model(comps, spec["propagator"])  # the parameters' values, for both passes
+        spec["versions"] = soa.versions()
         ox, oy, odx, ody, opl, zout, _, _, _ = _fwd_launch(comps, soa, packed=spec["packed"])
         spec["zout"] = zout
         ctx.spec = spec
@@ -280,7 +287,8 @@ class _TraceFn(torch.autograd.Function):
             ipl = torch.zeros(n, dtype=torch.float64, device=dev) if gpl is None else \
                 torch.empty(n, dtype=torch.float64, device=dev)
         need_raw = bool(plist) or spec["z_grad"]
-        m = spec["packed"][0]
+        # rays that changed in place since the forward: the parameters at their present values too
+        m, table = spec["packed"] if soa.versions() == spec["versions"] else pack_model(comps, spec["propagator"])
         raw = torch.empty((2 * len(comps), 4), dtype=torch.float64, device=dev) if need_raw else None
         ws = None
         if need_raw:
@@ -292,7 +300,7 @@ class _TraceFn(torch.autograd.Function):
                                      N.ptr(raw), N.ptr(ws), 0 if ws is None else ws.numel(),
                                      N.stream_ptr())
         N.check(st, "tg_trace_vjp_ex")
-        pgrads = param_gradients(comps, plist, raw) if plist else []
+        pgrads = param_gradients(comps, plist, raw, table) if plist else []
         gz = (-raw[0, 0]).reshape(()) if (spec["z_grad"] and len(comps)) else None
         shape = spec["shape"]
         rs = lambda t: None if t is None else t.reshape(shape)  # noqa: E731

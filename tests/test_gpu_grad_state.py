@@ -59,3 +59,47 @@ def test_field_gradients_are_the_forward_state_s(cuda, moved, astigmatic, dev):
     assert all(v.abs().max() > 0 and torch.isfinite(v.abs()).all() for v in want.values())
     for k, v in want.items():
         assert torch.equal(got[k], v), k
+
+
+def _trace(dev, moved):
+    import temgymcore_gb300 as t
+    r = np.random.default_rng(0)
+    n = 1001
+    rays = {k: torch.tensor(r.normal(0, 1e-3, n), dtype=torch.float32, device="cuda", requires_grad=True)
+            for k in ("x", "y", "dx", "dy")}
+    f, spx, spy = (torch.tensor(v, device=dev, **P64) for v in (0.25, 1e-4, 2e-4))
+    err = _descan_error(r, dev)
+    model = [t.Descanner(z=0.1, scan_pos_x=spx, scan_pos_y=spy, scan_tilt_x=1e-4, scan_tilt_y=3e-4, descan_error=err),
+             t.Lens(z=0.5, focal_length=f), t.Biprism(z=0.7, def_x=1e-4), t.Detector(z=1.3, **GRID)]
+    leaves = {**rays, "f": f, "spx": spx, "spy": spy, **err._asdict()}
+    early, late = moved
+    with torch.no_grad():
+        for k in early:
+            leaves[k].mul_(1.5)
+    out = t.run_to_end(t.Ray(z=0.0, pathlength=0.0, **rays), model)
+    with torch.no_grad():
+        for k in late:
+            leaves[k].mul_(1.5)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    up = [torch.randn(n, device="cuda", generator=g) for _ in range(4)]
+    return dict(zip(leaves, torch.autograd.grad([out.x, out.y, out.dx, out.dy], list(leaves.values()), up)))
+
+
+def _equal(got, want):
+    assert all(v.abs().max() > 0 for v in want.values())
+    for k, v in want.items():
+        assert torch.equal(got[k], v), k
+
+
+@pytest.mark.parametrize("dev", ["cpu", "cuda"])
+@pytest.mark.parametrize("moved", [("f",), ("spx", "spy"), ("pxo_pxi", "syo_pyi", "pyo_sxi"), ("f", "spy", "pxo_pyi")])
+def test_trace_gradients_with_moved_parameters_are_the_forward_state_s(cuda, moved, dev):
+    _equal(_trace(dev, ((), moved)), _trace(dev, ((), ())))
+
+
+@pytest.mark.parametrize("dev", ["cpu", "cuda"])
+@pytest.mark.parametrize("moved", [("x", "dy"), ("x", "f"), ("dx", "spx", "pxo_pxi")])
+def test_trace_gradients_with_moved_rays_are_the_present_state_s(cuda, moved, dev):
+    """The rays are not copied for the backward pass: where they moved, it reads
+    the parameters at their present values too."""
+    _equal(_trace(dev, ((), moved)), _trace(dev, (moved, ())))
