@@ -368,7 +368,10 @@ class _FieldFn(torch.autograd.Function):
     def forward(ctx, spec, *inputs):
         plan = spec["plan"]
         ctx.spec = spec
-        return plan.evaluate()  # the plan's own buffer: nothing else evaluates it
+        # the plan's own buffer, which the plan lets go: out.grad_fn holds the plan, and
+        # a plan that held out would keep both until the cyclic collector runs
+        out, plan.out = plan.evaluate(), None
+        return out
 
     @staticmethod
     def backward(ctx, grad):
