@@ -295,6 +295,10 @@ class FieldPlan:
             self._method = "separable" if int(self.flags.item()) == 0 else "direct"
         return self._method
 
+    @method.setter
+    def method(self, name: str) -> None:
+        self._method = name
+
     def evaluate(self, method: str | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
         o = self.out if out is None else out
         if method is None and self._method is None:
