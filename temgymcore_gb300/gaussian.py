@@ -185,12 +185,24 @@ class BeamSet:
     @property
     def wl(self) -> torch.Tensor:
         """Wavelength per beam."""
-        return torch.full_like(self.x, self.wl_scalar) if self._wl is None else self._wl
+        if self._wl is None:
+            self._wl = torch.full_like(self.x, self.wl_scalar)
+        return self._wl
+
+    @wl.setter
+    def wl(self, v: torch.Tensor) -> None:
+        self._wl = v
 
     @property
     def theta(self) -> torch.Tensor:
         """Rotation per beam."""
-        return torch.zeros_like(self.x) if self._theta is None else self._theta
+        if self._theta is None:
+            self._theta = torch.zeros_like(self.x)
+        return self._theta
+
+    @theta.setter
+    def theta(self, v: torch.Tensor) -> None:
+        self._theta = v
 
     def own(self) -> "BeamSet":
         """The same values in arrays that nothing else holds (an array already in
