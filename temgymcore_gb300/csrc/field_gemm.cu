@@ -314,13 +314,7 @@ int launch_field_gemm(const __nv_bfloat16_raw* vplanes, const __nv_bfloat16_raw*
   A.w = w;
   A.part = part;
   A.flags = flags;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_field_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem) !=
-        cudaSuccess)
-      return TG_ERR_CUDA;
-    attr = true;
-  }
+  if (smem_opt_in<k_field_gemm>(kGemmSmem) != cudaSuccess) return TG_ERR_CUDA;
   dim3 grid(lines_v / 128, lines_u / 128, splits);
   k_field_gemm<<<grid, 128, kGemmSmem, s>>>(maps, A);
   return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
