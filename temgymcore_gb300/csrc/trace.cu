@@ -472,13 +472,11 @@ static bool use_shared_hist(int64_t n, const tg_grid* grid) {
   return grid && use_shared_hist(n, grid->h, grid->w);
 }
 
-// Opt a shared-histogram kernel into the full shared-memory budget, once per
+// Opt a shared-histogram kernel into the full shared-memory budget, once per device and
 // instantiation (before any graph capture that replays it).
 template <auto Kernel>
 static cudaError_t shared_hist_attr() {
-  static cudaError_t done = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (kShMaxBins / 2) * (int)sizeof(uint32_t));
-  return done;
+  return smem_opt_in<Kernel>((kShMaxBins / 2) * (int)sizeof(uint32_t));
 }
 
 static size_t shared_hist_bytes(int64_t h, int64_t w) {
@@ -501,9 +499,7 @@ static int smem_optin() {
 // The prefetching shared-histogram kernel with the whole opt-in budget.
 template <auto Kernel>
 static cudaError_t prefetch_attr() {
-  static cudaError_t done =
-      cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin());
-  return done;
+  return smem_opt_in<Kernel>(smem_optin());
 }
 
 static int trace_fwd_impl(const tg_model* model, const tg_rays* in, tg_rays* out,

@@ -13,7 +13,7 @@ def _source(name):
         return fh.read()
 
 
-@pytest.mark.parametrize("name", ["field_gemm.cu"])
+@pytest.mark.parametrize("name", ["field_gemm.cu", "trace.cu"])
 def test_the_opt_in_is_kept_per_device(name):
     src = _source(name)
     assert "cudaFuncSetAttribute" not in src and "smem_opt_in<" in src
