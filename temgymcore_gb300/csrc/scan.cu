@@ -283,14 +283,27 @@ k_scan_hist(const __grid_constant__ Program P, const __grid_constant__ ScanArgs 
             __stcs(rows + i, v);
           }
         } else {
-          for (int64_t i = (int64_t)lo * W + threadIdx.x; i < (int64_t)hi * W; i += blockDim.x) {
-            const int row = (int)(i / W), c = (int)(i - (int64_t)row * W) - c0;
+          // A thread's row and column advance by the block's width in rows and
+          // columns.  (One division by W a pixel: 301 x 301 images, 625 probes of 64
+          // rays, 90 us in 32 bits, 127 in 64.)  h, w <= 65,535: fewer than 2^32 -
+          // 2^16 pixels.
+          const uint32_t total = (uint32_t)(hi - lo) * (uint32_t)W;
+          const int dr = kScanThreads / W, dc = kScanThreads - dr * W;
+          int row = lo + (int)threadIdx.x / W, c = (int)threadIdx.x % W - c0;
+          int32_t* px = img + (int64_t)lo * W;
+          for (uint32_t i = threadIdx.x; i < total; i += kScanThreads) {
             int v = 0;
             if (row >= b0 && row < b1 && c >= 0 && c < wc) {
               const int bin = (row - b0) * wc + c;
               v = (int)((win[bin >> 1] >> (16 * (bin & 1))) & 0xffffu);
             }
-            __stcs(img + i, v);
+            __stcs(px + i, v);
+            row += dr;
+            c += dc;
+            if (c >= W - c0) {
+              c -= W;
+              ++row;
+            }
           }
         }
         lo = hi;
