@@ -12,7 +12,8 @@
 //      keeps each ray's packed pixel in shared memory,
 //   3. reduces the hits' bounding box and histograms it in a shared-memory
 //      window, in bands of as many box rows as fit the window (one band in
-//      the usual case: a probe lights a small disc),
+//      the usual case: a probe lights a small disc; wider ones where that pays,
+//      ScanArgs::bands),
 //   4. writes the dense image once: the window rows, and a quarter of the
 //      image's rows of zeros around them, as 16-byte stores; the other rows
 //      are all zeros and leave as TMA bulk copies from a zero buffer in
@@ -20,8 +21,8 @@
 //      the copy engine streams them).  Both write paths run at once.
 // Small images and large bundles run k_scan_image instead (scan_use_image): the
 // probe's whole image as packed 16-bit counters in shared memory, written out
-// once.  What fits neither (an image beyond shared memory, more than 65,535
-// rays) takes the slow path: zero-fill, barrier, global atomics.  The HBM
+// once.  What takes neither (wide discs on a large image, more than 65,535 rays)
+// is zero-filled and counted with global atomics.  The HBM
 // traffic is therefore the dense histogram write, ~h*w*4 bytes/probe.
 #include <cstring>
 
@@ -34,6 +35,7 @@ namespace tg {
 constexpr int kScanThreads = 256;
 constexpr int kMaxSmemRays = 4096;  // packed pixels kept in shared memory
 constexpr int kZeroBytes = 8192;    // zero source of the bulk row copies
+constexpr int kSmallBox = 5632;     // bins of a box that always takes the window (one band)
 // k_scan_hist's shared memory (four CTAs fill an SM): the zero source, the
 // packed pixels, and the rest as the window's 16-bit counters (16,000 bins
 // beside 4,096 rays, 22,000 beside 1,024)
@@ -53,6 +55,7 @@ struct ScanArgs {
   int32_t vec_in;  // the bundle's arrays (and probe_xy's rows) are 16-byte aligned: four consecutive rays a thread
   int32_t bulk;  // images in device memory: zero rows as TMA bulk copies
   int32_t win_bins;    // k_scan_hist's window (16-bit counters)
+  int32_t bands;       // boxes above kSmallBox bins take the window up to this many twentieths of the rows
   int32_t store_rows;  // zero rows next to the window written by stores, not bulk copies
 };
 
@@ -216,7 +219,9 @@ k_scan_hist(const __grid_constant__ Program P, const __grid_constant__ ScanArgs 
     // window columns [c0, c0 + wc): whole groups of four pixels, so that a
     // group's counters are one aligned pair of words
     const int c0 = any ? cmin & ~3 : 0, wc = any ? ((cmax - c0) | 3) + 1 : 0;
-    if (fits && wc <= A.win_bins) {
+    const int rows_hit = any ? rmax - rmin + 1 : 0, cols_hit = any ? cmax - cmin + 1 : 0;
+    const bool small = (int64_t)rows_hit * cols_hit <= kSmallBox;
+    if (fits && wc <= A.win_bins && (small || rows_hit * 20 <= H * A.bands)) {
       // rows [r0, r1) are written by stores: the box rows and, with bulk
       // copies, store_rows zero rows around them; the rows outside are zeros:
       // bulk copies of the zero buffer (row starts are 16-byte aligned: W is a
@@ -312,7 +317,12 @@ k_scan_hist(const __grid_constant__ Program P, const __grid_constant__ ScanArgs 
       } while (any && b0 <= rmax);
     } else {
       // slow path: zero the image, then global atomics (re-trace if needed)
-      for (int64_t i = threadIdx.x; i < (int64_t)H * W; i += blockDim.x) img[i] = 0;
+      const int64_t total = (int64_t)H * W, odd = (int64_t)(-(reinterpret_cast<uintptr_t>(img) >> 2) & 3);
+      const int64_t head = odd < total ? odd : total, vecs = (total - head) >> 2;  // 16-byte stores from img + head on
+      int4* body = reinterpret_cast<int4*>(img + head);
+      for (int64_t i = threadIdx.x; i < vecs; i += kScanThreads) body[i] = make_int4(0, 0, 0, 0);
+      if (threadIdx.x < head) img[threadIdx.x] = 0;
+      if (threadIdx.x < total - head - 4 * vecs) img[head + 4 * vecs + threadIdx.x] = 0;
       __syncthreads();
       if (fits) {
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -477,9 +487,11 @@ extern "C" int tg_scan_hist(const tg_model* model, const tg_rays* bundle, const 
   // write paths run in parallel (256x256 images, 64x64 probes: 0.1815 ms with
   // bulk copies alone, 0.1777 ms with 64 stored rows; 32 and 80 rows between)
   A.store_rows = grid->h / 4;
+  bool on_host = false;
   {  // images may live in pinned host memory (written by the kernel across the host link)
     cudaPointerAttributes pa;
     if (cudaPointerGetAttributes(&pa, hist) != cudaSuccess) return TG_ERR_CUDA;
+    on_host = pa.type == cudaMemoryTypeHost;
     A.bulk = A.vec4 && pa.type == cudaMemoryTypeDevice;
     if (pa.type != cudaMemoryTypeDevice && pa.type != cudaMemoryTypeHost && pa.type != cudaMemoryTypeManaged)
       return TG_ERR_INVALID;  // unregistered host memory
@@ -504,6 +516,25 @@ extern "C" int tg_scan_hist(const tg_model* model, const tg_rays* bundle, const 
     per_sm = q > 0 ? q : 1;
   }
   int blocks = sm_count_scan() * per_sm;
+  // Larger boxes: a zero fill with a global atomic a hit, or the window in bands?
+  // The window leaves the zero rows to the bulk copies, which pays when every SM
+  // holds its four CTAs and enough rows are left to them.  The bands' time over the
+  // other's, 1,024 to 4,096 rays a probe:
+  //   200 x 200, 625-12,321 probes: 100 rows 0.85-1.05, 130 rows 1.0-1.2
+  //   256 x 256, 625-7,569:  130 rows 0.82-1.07, 160 rows 0.84-1.17, all rows 0.99-1.4
+  //   300 x 300, 625-5,476:  160 rows 0.76-0.93, 200 rows 0.79-1.0, all rows 0.95-1.13
+  //   512 x 512, 625-1,849:  300 rows 0.72-0.93, 400 rows 0.84-1.01, all rows 0.95-1.11
+  // with one CTA an SM (81 probes, 512 x 512) 1.1 for 100 rows, 1.9 for all, and for
+  // images of 160 x 160, which stay in L2, 1.1 to 1.6.  Rows of odd widths have no
+  // bulk copies (301 x 301, 625 probes: 1.3-1.6).  Images in host memory take the bands always:
+  // an atomic there crosses the host link.
+  const int64_t pixels = (int64_t)grid->h * grid->w;
+  if (on_host)
+    A.bands = 20;
+  else if (!A.bulk || scan->n_probes < blocks || pixels < 200 * 200)
+    A.bands = 0;
+  else
+    A.bands = pixels < 300 * 300 ? 12 : 15;
   if (blocks > scan->n_probes) blocks = scan->n_probes;
   k_scan_hist<<<blocks, kScanThreads, kHistSmem, s>>>(P, A, B);
   return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
