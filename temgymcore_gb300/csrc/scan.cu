@@ -142,16 +142,17 @@ __device__ __forceinline__ void trace_rays(const Program& P, const ScanArgs& A, 
     }
   }
   float x[R], y[R];
-  bool nonfinite[R];
+  bool live[R], nonfinite[R];
 #pragma unroll
   for (int k = 0; k < R; ++k) {
     x[k] = r[k].x;
     y[k] = r[k].y;
+    live[k] = i0 + k * step < n;
   }
-  bin_rays<R>(x, y, B, py, px, nonfinite);
+  bin_rays<R>(x, y, B, live, py, px, nonfinite);
 #pragma unroll
   for (int k = 0; k < R; ++k) {
-    const bool in = i0 + k * step < n;
+    const bool in = live[k];
     hit[k] = in && alive[k] && (unsigned)py[k] < (unsigned)A.h && (unsigned)px[k] < (unsigned)A.w;
     if (in && nonfinite[k]) atomicOr(&g_tg_err, TG_EW_NONFINITE);
   }

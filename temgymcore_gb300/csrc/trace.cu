@@ -213,12 +213,14 @@ __device__ __forceinline__ void fwd_rays(const Program& P, const FwdArgs& A, con
     }
     if (A.do_bin) {
       int pys[R], pxs[R];
-      bool nonfinite[R];
-      bin_rays<R>(x, y, B, pys, pxs, nonfinite);
+      bool live[R], nonfinite[R];
+#pragma unroll
+      for (int k = 0; k < R; ++k) live[k] = i0 + k * step < n;
+      bin_rays<R>(x, y, B, live, pys, pxs, nonfinite);
 #pragma unroll
       for (int k = 0; k < R; ++k) {
         const int py = pys[k], px = pxs[k];
-        const bool inr = (i0 + k * step < n);
+        const bool inr = live[k];
         if (inr && nonfinite[k]) atomicOr(&g_tg_err, TG_EW_NONFINITE);
         if (A.hist) {
           bool ok = inr && alive[k] && py >= 0 && py < A.h && px >= 0 && px < A.w;
@@ -390,8 +392,9 @@ k_bin(const __grid_constant__ BinArgs A, const __grid_constant__ BinCoef B) {
     const bool inr = i < A.n;
     const float x[1] = {inr ? A.x[i] : 0.f}, y[1] = {inr ? A.y[i] : 0.f};
     int pys[1], pxs[1];
+    const bool live[1] = {inr};
     bool nonfinite[1];
-    bin_rays<1>(x, y, B, pys, pxs, nonfinite);
+    bin_rays<1>(x, y, B, live, pys, pxs, nonfinite);
     const int py = pys[0], px = pxs[0];
     if (inr) {
       if (A.pix_y) A.pix_y[i] = py;
