@@ -254,6 +254,14 @@ constexpr int kPfBytes = 4 * kShThreads * 16;  // 64 KB
 
 constexpr int kFwdRays = 4;  // rays a thread traces together
 
+// Arrays of any alignment: up to this many rays an SM one ray a thread (32
+// registers, eight blocks an SM), which is quicker while the launch is a single
+// wave of latencies.  us, one / four rays a thread: 10,007 rays through three
+// components 2.2 / 3.3, with a 256 x 256 image 3.0 / 5.1; 100,003 rays, eight 3.2 / 3.9,
+// with an image 4.5 / 6.0; 200,000 rays, one 2.7 / 2.7, three 3.3 / 3.6, eight 4.3 / 4.3;
+// 300,001 rays, one 2.9 / 2.8, three 3.9 / 3.7, eight 5.3 / 4.4.
+constexpr int kFwdOneRays = 1536;
+
 // kVec: every array is 16-byte aligned, a thread takes R consecutive rays.
 // Else a thread's rays lie blockDim.x apart, so that each access of a warp is
 // one contiguous run whatever the arrays' alignment (an odd ray count in a
@@ -544,13 +552,14 @@ static int trace_fwd_impl(const tg_model* model, const tg_rays* in, tg_rays* out
              al16(A.oy) && al16(A.odx) && al16(A.ody);
   A.opl_vec = A.opl && al16(A.opl);
   A.pix_vec = (!pix_y || al16(pix_y)) && (!pix_x || al16(pix_x));
+  const bool one = !vec && A.n <= (int64_t)kFwdOneRays * sm_count();
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (hist && workspace && use_shared_hist(A.n, grid) && ws_bytes >= shared_hist_bytes(grid) &&
       (reinterpret_cast<uintptr_t>(workspace) & 15) == 0) {
     // one CTA of kShThreads per SM, the detector's packed counters in shared memory
     const int bins = grid->h * grid->w;
     const size_t smem = (size_t)((bins + 1) / 2) * sizeof(uint32_t);
-    const int64_t per = (int64_t)kShThreads * kFwdRays, need = (A.n + per - 1) / per;
+    const int64_t per = (int64_t)kShThreads * (one ? 1 : kFwdRays), need = (A.n + per - 1) / per;
     const int blocks = (int)(need < sm_count() ? need : sm_count());
     A.rows = reinterpret_cast<uint32_t*>(workspace);
     cudaError_t e = cudaSuccess;
@@ -572,6 +581,14 @@ static int trace_fwd_impl(const tg_model* model, const tg_rays* in, tg_rays* out
         e = shared_hist_attr<k_trace_fwd<kFwdRays, int, true, true>>();
         if (e == cudaSuccess) k_trace_fwd<kFwdRays, int, true, true><<<blocks, kShThreads, smem, s>>>(P, A, B);
       }
+    } else if (one) {
+      if (hist_i64) {
+        e = shared_hist_attr<k_trace_fwd<1, long long, false, true>>();
+        if (e == cudaSuccess) k_trace_fwd<1, long long, false, true><<<blocks, kShThreads, smem, s>>>(P, A, B);
+      } else {
+        e = shared_hist_attr<k_trace_fwd<1, int, false, true>>();
+        if (e == cudaSuccess) k_trace_fwd<1, int, false, true><<<blocks, kShThreads, smem, s>>>(P, A, B);
+      }
     } else {
       if (hist_i64) {
         e = shared_hist_attr<k_trace_fwd<kFwdRays, long long, false, true>>();
@@ -588,6 +605,12 @@ static int trace_fwd_impl(const tg_model* model, const tg_rays* in, tg_rays* out
     return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
   }
   const int threads = 256;
+  if (one) {  // a single wave (kFwdOneRays)
+    const unsigned blocks = (unsigned)((A.n + threads - 1) / threads);
+    if (hist_i64) k_trace_fwd<1, long long, false><<<blocks, threads, 0, s>>>(P, A, B);
+    else k_trace_fwd<1, int, false><<<blocks, threads, 0, s>>>(P, A, B);
+    return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
+  }
   const int64_t per = (int64_t)threads * kFwdRays, blocks_needed = (A.n + per - 1) / per;
   // every block resident at once: with the grid-stride loop each block has
   // the same share, so blocks waiting for a slot would lengthen the tail
