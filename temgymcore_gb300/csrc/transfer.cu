@@ -372,7 +372,14 @@ extern "C" int tg_transfer_rays(int64_t n, const double* rays, int32_t m, const 
     int64_t rows = (want + rblocks - 1) / rblocks;
     const int groups = (m + kTrPlanes - 1) / kTrPlanes;
     if (rows > groups) rows = groups;
-    const int per = (int)((groups + rows - 1) / rows) * kTrPlanes;
+    int per = (int)((groups + rows - 1) / rows) * kTrPlanes;
+    // Few rays: one plane a thread while a single wave holds every block, two up
+    // to half a wave.  us, one or two planes / four: 1 ray x 7 planes 2.9 / 5.0,
+    // 1,000 x 3 3.5 / 6.0, 1,000 x 61 4.3 / 7.4, 5,000 x 5 3.7 / 7.2, 20,000 x 7 6.2 / 8.2;
+    // 30,000 x 8 and 20,000 x 12 (472 of 608 blocks) as two 9.0 / 8.0.
+    const int64_t wave = (int64_t)sm_count_transfer() * kTrMinBlocks;
+    if (rblocks * m <= wave) per = 1;
+    else if (rblocks * ((m + 1) / 2) <= wave / 2) per = 2;
     const size_t smem = sizeof(double) * (kTrThreads / 32) * kTrWarpDoubles +
                         sizeof(ulonglong2) * kTrTab * (size_t)(per < m ? per : m);  // at most 70 KB
     const int smem_max = (int)(sizeof(double) * (kTrThreads / 32) * kTrWarpDoubles + sizeof(ulonglong2) * kTrTab * kMaxTransfer);

@@ -54,3 +54,19 @@ def test_a_sum_of_two_floats_is_rounded_to_nearest(cuda, full):
     assert np.array_equal(out[:, :2], rays[:, :2] + rays[:, 2:4])
     assert np.array_equal(out[:, 2:4], rays[:, 2:4])
     assert np.array_equal(out[:, 4], rays[:, 0] + rays[:, 2] if full else rays[:, 4])
+
+
+@pytest.mark.parametrize("n,m", [(1, 1), (257, 3), (38_912, 4), (38_913, 4), (5_000, 61), (8_000, 19), (8_000, 20)])
+def test_planes_a_thread(cuda, n, m):
+    """One, two or four planes a thread (by blocks): each plane of a stack is the
+    last of the stack's first planes alone, bit for bit."""
+    r = np.random.default_rng(n)
+    mats = r.normal(0, 0.6, (m, 5, 5))
+    mats[:, 4] = [0.0, 0.0, 0.0, 0.0, 1.0]
+    rays = r.normal(0, 1.0, (n, 5))
+    rays[:, 4] = 1.0
+    out = _out(rays, mats)
+    for p in {0, m // 2, m - 1}:
+        # result[k] is the product of the last k + 1 matrices
+        alone = np.concatenate([_out(rays[i:i + 500], mats[m - 1 - p:])[:, -1] for i in range(0, n, 500)])
+        assert np.array_equal(out[:, p], alone)
