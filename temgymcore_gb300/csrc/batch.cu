@@ -100,8 +100,8 @@ struct RecLayout {
   int D, D4, q, l, k, ev, total;
 };
 
-__host__ __device__ inline RecLayout rec_layout(int nb, int n_bip_ev, int n_ap_ev) {
-  RecLayout L;
+__host__ __device__ constexpr RecLayout rec_layout(int nb, int n_bip_ev, int n_ap_ev) {
+  RecLayout L{};
   L.D = 5 + nb;
   L.D4 = (L.D + 3) & ~3;
   L.q = 4 * L.D;
@@ -204,6 +204,9 @@ __device__ __forceinline__ void batch_prefetch(const BatchIO& io, const BTile& T
 // up to two biprisms only: 327).  Bound by instructions issued and the shared
 // memory reads of the records, at half occupancy (64 registers; 3 blocks of 80: 343).
 constexpr bool batch_pairs(int R, int nb) { return R >= 2 && nb >= 0; }
+// The largest record of a model whose tiles run in pairs (floats): all that a
+// launch ever holds twice over, whatever its other models' records.
+constexpr int kPairMaxRec = rec_layout(kRegBip, kRegBip, TG_MAX_COMPONENTS - kRegBip).total;
 
 // Two rays of a tile at a time (R >= 2, at most four biprisms), as batch_tile
 // forms each: the rays are the halves of packed pairs, the record is held twice
@@ -584,11 +587,16 @@ k_batch(const uint8_t* __restrict__ plan, const __grid_constant__ BatchIO io,
       continue;
     }
     const int nm = M.n_mom, nb = M.n_bip;
+    const bool twice = batch_pairs(R, nb <= kRegBip ? nb : -1);
+    if (twice && M.rec_floats > kPairMaxRec) {  // corrupt plan, as above
+      if (threadIdx.x == 0) atomicOr(&g_tg_err, TG_EW_TABLE);
+      __syncthreads();
+      continue;
+    }
     batch_prefetch<R>(io, T, pf_base, nf, adj, 0, 0);
     {
       const float4* src = reinterpret_cast<const float4*>(recs + M.rec_off);
       float4* dst = reinterpret_cast<float4*>(srec);
-      const bool twice = batch_pairs(R, nb <= kRegBip ? nb : -1);
       for (int i = threadIdx.x; i < (M.rec_floats >> 2); i += blockDim.x) {
         const float4 r = __ldg(src + i);
         if (twice) {
@@ -1081,7 +1089,10 @@ extern "C" int tg_batch_run(const void* plan_dev, const tg_batch_info* info, con
   if (tail > dyn) dyn = tail;
   dyn = (dyn + 15) & ~(size_t)15;
   const int rec_smem_off = (int)(dyn / sizeof(float));
-  dyn += ((size_t)info->max_record_floats * (rays_per_thread >= 2 ? 2 : 1) * sizeof(float) + 15) & ~(size_t)15;
+  // (a record held twice over is one of at most four biprisms)
+  size_t rec = (size_t)info->max_record_floats;
+  if (rays_per_thread >= 2) rec = std::max(rec, 2 * std::min(rec, (size_t)kPairMaxRec));
+  dyn += (rec * sizeof(float) + 15) & ~(size_t)15;
   const int pf_off = (int)(dyn / sizeof(float));
   dyn += (size_t)2 * (adj ? 6 : 4) * rays_per_thread * block * sizeof(float);
   if (dyn > 200 * 1024) return TG_ERR_TOO_LARGE;
