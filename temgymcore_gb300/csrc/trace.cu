@@ -1090,12 +1090,18 @@ __device__ __forceinline__ void lean_reverse(const Op& op, Ray4& r, Ray4& a, flo
 // evict-first loads and stores 0.157 ms (three blocks 0.189 ms).
 constexpr int kLeanRays = 8;    // rays per thread
 constexpr int kLeanBlocks = 2;  // resident blocks per SM (register bound)
-// Steps up to which a chain with every gradient given takes the short form, a
-// dispatch per ray and step: slower code, but two components are bound by memory,
-// where the quicker form mixes the blocks' reads and writes more.  Lens + Detector,
-// short / quick: 2 M rays 24.9 / 25.8 us, 8 M 71.1 / 73.1, 16.8 M 127.8 / 135.4
-// (130 with a barrier a turn); three components, 16.8 M: 141 / 131.
-constexpr int kLeanShort = 4;
+// The short form, a dispatch per ray and step, for chains with every gradient
+// given: slower code, but short chains are bound by memory, where the quicker form
+// mixes the blocks' reads and writes more.  us, short / quick:
+//   two components   2 M rays 24.9 / 25.8, 8 M 71.1 / 73.1, 16.8 M 123-128 / 130-135
+//   three, no sums   0.3 M 5.7 / 5.4, 1 M 10.6 / 11.5, 4 M 32.9 / 33.6, 16.8 M 119.9 / 123.0
+//   three, sums      0.3 M 9.5 / 9.5, 0.5 M 11.1 / 11.6, 1 M 15.7 / 16.2, 2 M 24.3 / 24.2, 16.8 M 134 / 127
+//   four, no sums    0.3 M 6.4 / 6.2, 1 M 12.8 / 13.5, 1.5 M 17.3 / 17.1;  sums 1 M 18.5 / 18.2
+// (16.8 M rays and two components: 130 with a barrier a turn).
+static bool lean_short(int n_steps, bool sums, int64_t n) {
+  const bool window = n > 400000 && n < 1250000;
+  return n_steps <= 4 || (n_steps <= 6 && (!sums || window)) || (n_steps <= 8 && !sums && window);
+}
 
 // One component at a time, its kind decided once for all R rays of a thread (both
 // ways: its free-space step and its own; kShort: step by step).  The sums run in
@@ -1333,7 +1339,7 @@ static int trace_vjp_impl(const tg_model* model, const tg_rays* in, const tg_ray
   if (lean) {
     const size_t smem = sizeof(float) * (kVjpThreads / 32) * 4 * (size_t)P.n_steps;  // at most 15 KB
     const size_t dyn = A.partial ? smem : 0;
-    if (P.n_steps <= kLeanShort && !opt)
+    if (!opt && lean_short(P.n_steps, A.partial != nullptr, A.n))
       k_trace_vjp_lean<kLeanRays, true><<<grid, kVjpThreads, dyn, s>>>(P, A);
     else
       k_trace_vjp_lean<kLeanRays, false><<<grid, kVjpThreads, dyn, s>>>(P, A);
