@@ -190,6 +190,7 @@ k_field_gemm(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gemm
   const int row0 = mt * 128 + warp * 32, rows = A.h - row0 < 32 ? A.h - row0 : 32;
   const bool even = (A.w & 1) == 0;  // every row starts on 16 bytes
   for (int c = 0; c < 4; ++c, mine += 32 * kEpiPitch) {
+    if (rows <= 0 || nt * 128 + c * 32 >= A.w) break;  // the whole warp: nothing of the image here
     uint32_t a_re[32], a_im[32], b_re[32], b_im[32];
     tmem_ld32(tmem + lane_base + 0 + c * 32, a_re);    // D0: Vr Ur
     tmem_ld32(tmem + lane_base + 128 + c * 32, a_im);  // D0: Vr Ui
