@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import dataclasses
 from dataclasses import dataclass, field
+from math import isfinite
 from typing import Any, NamedTuple
 
 import numpy as np
@@ -25,6 +26,12 @@ def _f(v) -> float:
     if isinstance(v, torch.Tensor):
         return float(v.item())
     return float(v)
+
+
+def _numbers(v) -> bool:
+    """True for a tuple of two finite Python numbers."""
+    return (type(v) is tuple and len(v) == 2 and type(v[0]) in (int, float) and type(v[1]) in (int, float)
+            and isfinite(v[0]) and isfinite(v[1]))
 
 
 class Component(HasParamsMixin):
@@ -193,6 +200,15 @@ class Grid:
 
     def _pixel_map(self) -> tuple:
         """The six numbers of the pixels -> metres map (y row, then x row)."""
+        ps, sh, ce = self.pixel_size, self.shape, self.centre
+        if (type(self).pixels_to_metres_mat is Grid.pixels_to_metres_mat and _numbers(ps) and _numbers(sh)
+                and _numbers(ce) and ce[0] == 0 and ce[1] == 0 and type(self.rotation) in (int, float)
+                and self.rotation == 0):
+            # on the axis and not turned: one product an entry, rounded as the
+            # matrices' product rounds it (ten times the host time)
+            py, px = float(ps[0]), float(ps[1])
+            vy = py if self.flip_y else -py
+            return (vy, 0.0, vy * (-(float(sh[0]) - 1.0) / 2.0), 0.0, px, px * (-(float(sh[1]) - 1.0) / 2.0))
         m = self.pixels_to_metres_mat
         return tuple(float(v) for v in (m[0, 0], m[0, 1], m[0, 2], m[1, 0], m[1, 1], m[1, 2]))
 

@@ -74,3 +74,26 @@ def test_the_number_of_beams_follows_the_fields():
         for k, v in beams(7).items():
             object.__setattr__(r, k, v)
         assert r.size == 7
+
+
+@pytest.mark.parametrize("flip", [False, True])
+@pytest.mark.parametrize("centre", [(0.0, 0.0), (0, 0), (1e-6, -2e-6), [0.0, 0.0], (np.float64(0.0), 0.0)])
+@pytest.mark.parametrize("rotation", [0.0, 0, 30.0, torch.tensor(0.0), np.float32(0.0)])
+def test_the_pixel_map_is_the_matrices_product(centre, rotation, flip):
+    r = np.random.default_rng(0)
+    for shape in ((1, 1), (8, 9), (256, 255), (4096, 3)):
+        ps = tuple(float(v) for v in r.uniform(1e-7, 1e-3, 2))
+        det = t.Detector(z=1.0, pixel_size=ps, shape=shape, rotation=rotation, centre=centre, flip_y=flip)
+        m = det.pixels_to_metres_mat
+        assert det._pixel_map() == (m[0, 0], m[0, 1], m[0, 2], m[1, 0], m[1, 1], m[1, 2])
+
+
+def test_a_grid_with_its_own_map():
+    class Shifted(t.Detector):
+        @property
+        def pixels_to_metres_mat(self):
+            return super().pixels_to_metres_mat + 1e-3
+
+    det = Shifted(z=1.0, pixel_size=(1e-5, 1e-5), shape=(8, 9))
+    m = det.pixels_to_metres_mat
+    assert det._pixel_map() == (m[0, 0], m[0, 1], m[0, 2], m[1, 0], m[1, 1], m[1, 2])
