@@ -619,9 +619,9 @@ int tg_field_prep(const tg_model *model, const tg_beams *beams, const tg_pixel_m
                   void *workspace, size_t ws_bytes, int32_t *flags, void *stream);
 
 /* tg_field_prep that also writes what the adjoint starts from, the records of
- * the beams at unit amplitude, into unit (device, 16-byte aligned,
- * tg_field_unit_bytes(n) bytes): tg_field_vjp_steps then need not repeat the
- * preparation. */
+ * the beams at unit amplitude and the beams themselves, into unit (device,
+ * 16-byte aligned, tg_field_unit_bytes(n) bytes): tg_field_vjp_steps then need
+ * not repeat the preparation. */
 size_t tg_field_unit_bytes(int64_t n_beams);
 int tg_field_prep_grad(const tg_model *model, const tg_beams *beams, const tg_pixel_map *pm,
                        void *workspace, size_t ws_bytes, int32_t *flags, void *unit, size_t unit_bytes,
@@ -723,8 +723,9 @@ int tg_field_vjp_ex(int32_t method, const tg_model *model, const tg_beams *beams
                     void *stream);
 /* tg_field_vjp_ex that forms only the entries of out->raw whose byte in
  * want [2 * n_components][4] (host; NULL = all) is not 0; the others are 0.
- * unit: the records that tg_field_prep_grad wrote for the same model, beams and
- * pixel map (device, 16-byte aligned), or NULL to have them formed here. */
+ * unit: what tg_field_prep_grad wrote for the same model, beams and pixel map
+ * (device, 16-byte aligned), or NULL to have it formed here.  With it the beams
+ * are those that the preparation saw: the arrays of beams are not read. */
 int tg_field_vjp_steps(int32_t method, const tg_model *model, const tg_beams *beams, const tg_pixel_map *pm,
                        const float *grad, const tg_field_grads *out, const unsigned char *want,
                        const void *unit, void *workspace, size_t ws_bytes, void *stream);

@@ -332,6 +332,27 @@ k_field_prep(const __grid_constant__ DModel M, const __grid_constant__ PrepArgs 
   if (k_rc.re != 0.0 || k_rc.im != 0.0) atomicOr(A.flags, 1);
 }
 
+// The beams into the buffer of the unit records (KeptBeams).  A kernel of its own
+// (2 us at 8,192 beams): with these stores in k_field_prep the compiler contracts
+// its float64 expressions anew, and the records move by an ulp.
+__global__ void __launch_bounds__(256) k_field_keep(const __grid_constant__ PrepArgs A, const KeptBeams K) {
+  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= A.n) return;
+  K.x[b] = A.x[b];
+  K.y[b] = A.y[b];
+  K.dx[b] = A.dx[b];
+  K.dy[b] = A.dy[b];
+  K.pl[b] = A.pl[b];
+  K.wl[b] = A.wl ? A.wl[b] : A.wl_scalar;
+  K.theta[b] = A.theta ? A.theta[b] : 0.0;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    K.waist[2 * b + j] = A.waist[2 * b + j];
+    K.radii[2 * b + j] = A.radii[2 * b + j];
+    K.amp[2 * b + j] = A.amp[2 * b + j];
+  }
+}
+
 // The preparation's status word decides on the device which of the two methods'
 // kernels work (tg_field_eval_auto launches both): a kernel of the other method
 // returns at once.  No flag: no decision.
@@ -909,6 +930,7 @@ static int field_prep_launch(const DModel& dm, const tg_beams* beams, const tg_p
   // spread the (float64-bound) beams over every SM
   int blocks = (int)((beams->n + 63) / 64);
   k_field_prep<<<blocks, 64, 0, s>>>(dm, A);
+  if (unit) k_field_keep<<<(unsigned)((beams->n + 255) / 256), 256, 0, s>>>(A, kept_beams(unit, beams->n));
   return cudaGetLastError() == cudaSuccess ? TG_OK : TG_ERR_CUDA;
 }
 }  // namespace tg
@@ -936,7 +958,7 @@ extern "C" int tg_field_prep(const tg_model* model, const tg_beams* beams,
 }
 
 extern "C" size_t tg_field_unit_bytes(int64_t n_beams) {
-  return n_beams > 0 ? (size_t)n_beams * sizeof(BeamFast) : 0;
+  return n_beams > 0 ? (size_t)n_beams * kKeptBytes : 0;
 }
 
 extern "C" int tg_field_prep_grad(const tg_model* model, const tg_beams* beams, const tg_pixel_map* pm,

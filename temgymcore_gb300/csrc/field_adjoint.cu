@@ -1149,7 +1149,9 @@ static int field_vjp_impl(const tg_model* model, const tg_beams* beams, const tg
   if (out->raw && cudaMemsetAsync(out->raw, 0, sizeof(double) * 4 * (size_t)nsteps, s) != cudaSuccess)
     return TG_ERR_CUDA;
   if (n == 0) return TG_OK;
-  // 1. unit-amplitude records, unless the forward preparation left them
+  // 1. unit-amplitude records, unless the forward preparation left them (and the
+  // beams that they belong to)
+  const bool left = unit != nullptr;
   if (!unit) {
     int st = field_prep_unit_amp(dm, beams, pm, ws + L.rec, field_records_bytes(n), stream, input_plane ? 1 : 0);
     if (st != TG_OK) return st;
@@ -1232,6 +1234,16 @@ static int field_vjp_impl(const tg_model* model, const tg_beams* beams, const tg
     B.wl = beams->wavelength;
     B.wl_scalar = beams->wavelength_scalar;
     B.theta = beams->theta;
+    if (left) {
+      const KeptBeams k = kept_beams(const_cast<void*>(unit), n);  // read only
+      B.x = k.x; B.y = k.y; B.dx = k.dx; B.dy = k.dy;
+      B.pl = k.pl;
+      B.amp = k.amp;
+      B.waist = k.waist;
+      B.radii = k.radii;
+      B.wl = k.wl;
+      B.theta = k.theta;
+    }
     B.pm.h = pm->h;
     B.pm.w = pm->w;
     for (int i = 0; i < 6; ++i) B.pm.t[i] = pm->t[i];

@@ -62,6 +62,20 @@ struct alignas(16) BeamFast {
   float rho_re, rho_im;  // exp(-2 b_cc + i 2pi (2 p_cc)): column-step ratio of ratios
 };
 
+// The beams as the differentiable preparation saw them, behind its unit records
+// in the same buffer: the adjoint's chain rule then belongs to the same values
+// as the records, whatever has become of the caller's arrays.
+struct KeptBeams {
+  double *x, *y, *dx, *dy, *pl, *waist, *radii, *wl, *theta;  // waist and radii in pairs
+  float* amp;                                                // in pairs
+};
+constexpr size_t kKeptBytes = sizeof(BeamFast) + 11 * sizeof(double) + 2 * sizeof(float);  // a beam
+inline KeptBeams kept_beams(void* unit, int64_t n) {
+  double* d = reinterpret_cast<double*>(reinterpret_cast<char*>(unit) + n * sizeof(BeamFast));
+  return KeptBeams{d,         d + n,     d + 2 * n, d + 3 * n,  d + 4 * n,
+                   d + 5 * n, d + 7 * n, d + 9 * n, d + 10 * n, reinterpret_cast<float*>(d + 11 * n)};
+}
+
 // float64 record for the all-float64 comparator kernel, 128 bytes.
 struct alignas(16) BeamF64 {
   double re[6];   // c_cc, c_rr, c_rc, c_c, c_r, c_0 real parts (radians)

@@ -204,19 +204,6 @@ class BeamSet:
     def theta(self, v: torch.Tensor) -> None:
         self._theta = v
 
-    def own(self) -> "BeamSet":
-        """The same values in arrays that nothing else holds (an array already in
-        the kernel layout is the caller's own until then)."""
-        parts = [t for t in (self.x, self.y, self.dx, self.dy, self.pl, self.waist, self.radii, self._wl, self._theta)
-                 if t is not None]
-        flat = [t.reshape(-1) for t in parts]
-        own = iter(torch.cat(flat).split([t.numel() for t in flat]))
-        self.x, self.y, self.dx, self.dy, self.pl = (next(own) for _ in range(5))
-        self.waist, self.radii = next(own).view(self.n, 2), next(own).view(self.n, 2)
-        self._wl, self._theta = (None if t is None else next(own) for t in (self._wl, self._theta))
-        self.amp = self.amp.clone()
-        return self
-
     def struct(self) -> TgBeams:
         b = TgBeams()
         b.n = self.n
@@ -275,9 +262,9 @@ class FieldPlan:
             packed = pack_model(comps)
             if _unit and self.beams.n:
                 # The records that the adjoint starts from, in the same pass.  Its chain
-                # rule has to see the same beams and model: both are kept as they are now.
+                # rule has to see the same beams and model: the preparation leaves a copy
+                # of the beams behind the records, and the packed model is kept.
                 self._packed = packed
-                self.beams.own()
             args = (C.byref(packed[0]), C.byref(self.beams.struct()), C.byref(self.pm), self.ws_ptr, self.ws_bytes,
                     self.flags.data_ptr())
             if self._packed is not None:
