@@ -23,6 +23,8 @@ from .tree_utils import HasParamsMixin
 
 
 def _f(v) -> float:
+    if type(v) is float:
+        return v
     if isinstance(v, torch.Tensor):
         return float(v.item())
     return float(v)
@@ -54,8 +56,8 @@ class Component(HasParamsMixin):
         comp.kind = self._kind
         comp.flags = 0
         comp.z = _f(self.z)
-        for i, v in enumerate(self._params()):
-            comp.p[i] = v
+        p = list(self._params())
+        comp.p[:len(p)] = p
 
     def new_with(self, **kw):
         """tree_utils.py:168-172."""
@@ -200,15 +202,21 @@ class Grid:
 
     def _pixel_map(self) -> tuple:
         """The six numbers of the pixels -> metres map (y row, then x row)."""
-        ps, sh, ce = self.pixel_size, self.shape, self.centre
-        if (type(self).pixels_to_metres_mat is Grid.pixels_to_metres_mat and _numbers(ps) and _numbers(sh)
-                and _numbers(ce) and ce[0] == 0 and ce[1] == 0 and type(self.rotation) in (int, float)
-                and self.rotation == 0):
-            # on the axis and not turned: one product an entry, rounded as the
-            # matrices' product rounds it (ten times the host time)
+        ps, sh, ce, rot = self.pixel_size, self.shape, self.centre, self.rotation
+        if (_numbers(ps) and _numbers(sh) and _numbers(ce) and ce[0] == 0 and ce[1] == 0 and type(rot) in (int, float)
+                and type(self).pixels_to_metres_mat is Grid.pixels_to_metres_mat):
+            # Centred on the axis: every factor up to the last is one product an
+            # entry, formed here without the matrices (a tenth of the host time, the
+            # same bits); a turned grid's last factor sums two and stays a matrix.
             py, px = float(ps[0]), float(ps[1])
-            vy = py if self.flip_y else -py
-            return (vy, 0.0, vy * (-(float(sh[0]) - 1.0) / 2.0), 0.0, px, px * (-(float(sh[1]) - 1.0) / 2.0))
+            up = 1.0 if self.flip_y else -1.0
+            oy, ox = -(float(sh[0]) - 1.0) / 2.0, -(float(sh[1]) - 1.0) / 2.0
+            if rot == 0:
+                return (up * py, 0.0, up * py * oy, 0.0, px, px * ox)
+            c, s = np.cos(np.pi / 180 * float(rot)), np.sin(np.pi / 180 * float(rot))
+            m = (np.array([[up * c * py, up * s * px, 0.0], [-s * py, c * px, 0.0], [0.0, 0.0, 1.0]])
+                 @ np.array([[1.0, 0.0, oy], [0.0, 1.0, ox], [0.0, 0.0, 1.0]]))
+            return (float(m[0, 0]), float(m[0, 1]), float(m[0, 2]), float(m[1, 0]), float(m[1, 1]), float(m[1, 2]))
         m = self.pixels_to_metres_mat
         return tuple(float(v) for v in (m[0, 0], m[0, 1], m[0, 2], m[1, 0], m[1, 1], m[1, 2]))
 

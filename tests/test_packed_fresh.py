@@ -78,7 +78,7 @@ def test_the_number_of_beams_follows_the_fields():
 
 @pytest.mark.parametrize("flip", [False, True])
 @pytest.mark.parametrize("centre", [(0.0, 0.0), (0, 0), (1e-6, -2e-6), [0.0, 0.0], (np.float64(0.0), 0.0)])
-@pytest.mark.parametrize("rotation", [0.0, 0, 30.0, torch.tensor(0.0), np.float32(0.0)])
+@pytest.mark.parametrize("rotation", [0.0, 0, 30.0, 45, -17.3, 359.9, 1e5, torch.tensor(0.0), np.float32(0.0)])
 def test_the_pixel_map_is_the_matrices_product(centre, rotation, flip):
     r = np.random.default_rng(0)
     for shape in ((1, 1), (8, 9), (256, 255), (4096, 3)):
