@@ -1118,8 +1118,11 @@ extern "C" int tg_batch_run(const void* plan_dev, const tg_batch_info* info, con
 // One call for callers that do not keep a plan: pack the models on the host,
 // copy the plan into the front of the caller's workspace (a synchronous
 // staging copy from pageable memory, so this entry point is not for graph
-// capture: tg_batch_plan + tg_batch_run are) and run with the launch shape
-// measured best on GB300 (tiles of 4,096 rays, 256 threads x 2 rays).
+// capture: tg_batch_plan + tg_batch_run are) and run with one fixed launch shape,
+// tiles of 4,096 rays, 256 threads x 2 rays: on 512 models (22-24 M rays) 305 and
+// 313 us, 336 and 302 with 16,384 x 512 x 2, 321 and 335 with 2,048 x 256 x 2 (which
+// sweeps of fewer than a hundred models prefer: 32 us against 36).  No shape is
+// best everywhere; callers with a sweep to repeat tune theirs.
 namespace tg {
 constexpr int32_t kDefTile = 4096, kDefBlock = 256, kDefRpt = 2;
 }
