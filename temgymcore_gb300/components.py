@@ -9,6 +9,7 @@ tensors receive gradients through the adjoint kernel).
 from __future__ import annotations
 
 import dataclasses
+import struct
 from dataclasses import dataclass, field
 from math import isfinite
 from typing import Any, NamedTuple
@@ -28,6 +29,10 @@ def _f(v) -> float:
     if isinstance(v, torch.Tensor):
         return float(v.item())
     return float(v)
+
+
+# TgComponent's first fields and n parameters as one write
+_FILL = [struct.Struct(f"=iid{n}d") for n in range(33)]
 
 
 def _numbers(v) -> bool:
@@ -53,11 +58,12 @@ class Component(HasParamsMixin):
         return [_f(getattr(self, n)) for n in self._pfields]
 
     def _pack(self, comp: N.TgComponent) -> None:
-        comp.kind = self._kind
-        comp.flags = 0
-        comp.z = _f(self.z)
-        p = list(self._params())
-        comp.p[:len(p)] = p
+        p = self._params()
+        if type(p) is not list or len(p) >= len(_FILL):
+            p = list(p)
+            comp.p[:len(p)] = p
+            p = ()
+        _FILL[len(p)].pack_into(comp, 0, self._kind, 0, _f(self.z), *p)  # kind, flags, z, p
 
     def new_with(self, **kw):
         """tree_utils.py:168-172."""
@@ -213,10 +219,10 @@ class Grid:
             oy, ox = -(float(sh[0]) - 1.0) / 2.0, -(float(sh[1]) - 1.0) / 2.0
             if rot == 0:
                 return (up * py, 0.0, up * py * oy, 0.0, px, px * ox)
-            c, s = np.cos(np.pi / 180 * float(rot)), np.sin(np.pi / 180 * float(rot))
-            m = (np.array([[up * c * py, up * s * px, 0.0], [-s * py, c * px, 0.0], [0.0, 0.0, 1.0]])
-                 @ np.array([[1.0, 0.0, oy], [0.0, 1.0, ox], [0.0, 0.0, 1.0]]))
-            return (float(m[0, 0]), float(m[0, 1]), float(m[0, 2]), float(m[1, 0]), float(m[1, 1]), float(m[1, 2]))
+            c, s = float(np.cos(np.pi / 180 * float(rot))), float(np.sin(np.pi / 180 * float(rot)))
+            m = (np.array((up * c * py, up * s * px, 0.0, -s * py, c * px, 0.0, 0.0, 0.0, 1.0)).reshape(3, 3)
+                 @ np.array((1.0, 0.0, oy, 0.0, 1.0, ox, 0.0, 0.0, 1.0)).reshape(3, 3)).tolist()
+            return (*m[0], *m[1])
         m = self.pixels_to_metres_mat
         return tuple(float(v) for v in (m[0, 0], m[0, 1], m[0, 2], m[1, 0], m[1, 1], m[1, 2]))
 
